@@ -66,8 +66,11 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t n, const FastDiv &f)
 }
 
 // J-line kernels: lanes of one warp share a line and stage its rows through
-// registers (k_jline), or one lane runs a whole line (k_jline_thread).
-enum LineKind : int { LK_WARP = 0, LK_THREAD = 1 };
+// shared memory (k_jline) or keep them in registers (k_jline_reg), or one lane
+// runs a whole line (k_jline_thread).
+enum LineKind : int { LK_WARP = 0, LK_THREAD = 1, LK_REG = 2 };
+constexpr int REG_PASSES = 2;     // k_jline_reg: passes over a line at most
+constexpr int REG_MIN_LANES = 4;  // and lanes per line at least
 
 // One system of the batch.
 struct SysDev {
@@ -76,7 +79,7 @@ struct SysDev {
     // Layout of the arrays in the form's working precision.  The FP64 drop-in
     // works on the caller's arrays (line pitch JMAX2, n cells).  The mixed form's
     // FP32 arrays (diagonals, factors, vectors) are its own: each J-line padded to
-    // a pitch that is a multiple of four cells, so every line starts on a 16-byte
+    // a pitch that is a multiple of eight cells, so every line starts on a 32-byte
     // boundary; the pad cells hold zeros (diagonal A(0) = 1).
     int cyc;             // cyclic axes (1 I, 2 J, 4 K): the interior cells' neighbours wrap
     int jp;              // line pitch of those arrays
@@ -91,6 +94,7 @@ struct SysDev {
     int lane_group;      // G: lanes that share one J-line (power of two <= 32)
     int line_kind;       // LineKind: which J-line kernel sweeps this system's lines
     int rows_per_lane;   // c: rows of a line each lane owns (G*c >= jmax2)
+    int line_np;         // LK_REG: full passes of G row chunks over the line
     int half_lines;      // ceil(imax2/2): parity-wave slots per k row
     double *a64;         // 7*n diagonals, Fortran A_M(DIMENSION_3,-3:3) order
     double *b64;         // B_M(:,M)

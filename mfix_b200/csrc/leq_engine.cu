@@ -30,7 +30,7 @@ static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 namespace {
 struct TuneTable {
     std::mutex mu;
-    std::map<std::pair<int, int>, int> lanes;  // (element bytes, line length) -> lanes per line
+    std::map<std::pair<int, int>, int> lanes;  // (element bytes, line length) -> line shape (set_shape)
     std::string path;
 };
 TuneTable &tunes()
@@ -39,20 +39,6 @@ TuneTable &tunes()
     return t;
 }
 }  // namespace
-
-// Lanes per J-line: the smallest power of two that leaves at most 12 rows per
-// lane (at most 32 lanes); rows per lane rounded up to odd so that lanes reading row t
-// of their chunks hit distinct shared-memory banks.
-void line_shape(int L, int *G, int *c)
-{
-    int g = 1;
-    while (g < 32 && g * 12 < L) g *= 2;
-    int cc = (L + g - 1) / g;
-    if (cc < 1) cc = 1;
-    if ((cc & 1) == 0) ++cc;
-    *G = g;
-    *c = g == 1 ? 1 : cc;  // one lane per line stages nothing
-}
 
 void *DeviceArena::take(size_t bytes)
 {
@@ -235,8 +221,8 @@ cudaError_t Engine::stage_close() { return cudaEventRecord(stage_ev_[stage_cur_]
 // form's precision), then the per-line flags; the mixed form's copy of the
 // initial guess follows that region.
 // Line pitch and cells of a system's arrays in the form's precision: the mixed
-// form's FP32 arrays pad each J-line to a multiple of four cells.
-int form_pitch(int jmax2, int precision) { return precision == PREC_MIXED ? (jmax2 + 3) / 4 * 4 : jmax2; }
+// form's FP32 arrays pad each J-line to a multiple of eight cells.
+int form_pitch(int jmax2, int precision) { return precision == PREC_MIXED ? (jmax2 + 7) / 8 * 8 : jmax2; }
 int64_t form_cells(int64_t n, int64_t lines, int precision)
 {
     if (precision != PREC_MIXED || lines <= 0) return n;
@@ -334,7 +320,7 @@ int Engine::setup_batch(const std::vector<SystemSpec> &specs, const SolveOptions
         d.ntiles = (int)((std::max(sp.n, d.np) + TILE_CELLS - 1) / TILE_CELLS);
         d.tile_base = tile_base;
         tile_base += d.ntiles;
-        shape_for(sp.jmax2, mixed ? 4 : 8, opt.force_lanes, &d.lane_group, &d.rows_per_lane, &d.line_kind);
+        shape_for(d, mixed ? 4 : 8, opt.force_lanes);
         d.half_lines = (sp.imax2 + 1) / 2;
         d.div_h = make_fastdiv((uint32_t)d.half_lines);
         d.a64 = sp.a;
@@ -428,30 +414,39 @@ int Engine::setup_batch(const std::vector<SystemSpec> &specs, const SolveOptions
 // keeps the line work of the systems with that line length only (autotuning).
 int Engine::configure_lines(int elem, int only_L)
 {
-    h_prefix_.assign(nsys_ + 1, 0);
+    // two lists of work items, so that neither kind of kernel walks past the other's:
+    // list 0 the systems of k_jline and k_jline_thread, list 1 those of k_jline_reg
+    const int lists = nsys_ + 1;
+    h_prefix_.assign(2 * (size_t)lists, 0);
     int cmax = 1;
     for (int s = 0; s < nsys_; ++s) {
         const SysDev &d = h_sys_[s];
-        cmax = std::max(cmax, d.rows_per_lane);
+        if (d.line_kind == LK_WARP) cmax = std::max(cmax, d.rows_per_lane);
         const int lpw = 32 / d.lane_group;
         const bool tuned = only_L < 0 && std::find(tune_lengths_.begin(), tune_lengths_.end(), d.jmax2) !=
                                                 tune_lengths_.end();
         const bool keep = d.n > 0 && (only_L == 0 || d.jmax2 == only_L || tuned);  // n = 0: empty slot of a live batch
         const int64_t slots = keep ? (int64_t)d.half_lines * d.kmax2 : 0;
-        h_prefix_[s + 1] = h_prefix_[s] + (int)((slots + lpw - 1) / lpw);
+        const int n = (int)((slots + lpw - 1) / lpw), mine = d.line_kind == LK_REG;
+        for (int q = 0; q < 2; ++q) h_prefix_[q * lists + s + 1] = h_prefix_[q * lists + s] + (q == mine ? n : 0);
     }
-    h_line_sys_.resize(std::max(h_prefix_[nsys_], 1));
-    for (int s = 0; s < nsys_; ++s)
-        std::fill(h_line_sys_.begin() + h_prefix_[s], h_line_sys_.begin() + h_prefix_[s + 1], s);
+    const int items = h_prefix_[nsys_], reg_items = h_prefix_[lists + nsys_];
+    h_line_sys_.resize(std::max(items + reg_items, 1));
+    for (int q = 0; q < 2; ++q) {
+        const auto at = h_line_sys_.begin() + (q ? items : 0);
+        for (int s = 0; s < nsys_; ++s) std::fill(at + h_prefix_[q * lists + s], at + h_prefix_[q * lists + s + 1], s);
+    }
     CK(stage_open(sizeof(SysDev) * h_sys_.size() + sizeof(int) * (h_prefix_.size() + h_line_sys_.size()) + 256));
     CK(upload_staged(&d_sys_, &sys_cap_, h_sys_.data(), h_sys_.size()));
     CK(upload_staged(&d_prefix_, &prefix_cap_, h_prefix_.data(), h_prefix_.size()));
-    CK(upload_staged(&d_line_sys_, &line_sys_cap_, h_line_sys_.data(), (size_t)h_prefix_[nsys_]));
+    CK(upload_staged(&d_line_sys_, &line_sys_cap_, h_line_sys_.data(), (size_t)(items + reg_items)));
     CK(stage_close());
     // the uploads may have (re)allocated the tables: the kernels' view follows them
     view_.sys = d_sys_;
     view_.line_prefix = d_prefix_;
     view_.line_sys = d_line_sys_;
+    view_.reg_prefix = d_prefix_ + lists;
+    view_.reg_sys = d_line_sys_ + items;
     if (!view_.sys || !view_.st || !view_.tiles || !view_.line_prefix || !view_.line_sys || !view_.partials)
         return fail("internal: batch tables missing on the device", -13);
     cfg_.line_cmax = cmax;
@@ -459,19 +454,20 @@ int Engine::configure_lines(int elem, int only_L)
     const int bpsm = elem == 4 ? prepare_line_kernel<float>(cmax, &wpb) : prepare_line_kernel<double>(cmax, &wpb);
     if (bpsm <= 0) return fail("J-lines too long for the shared-memory staging of the line kernel", -10);
     cfg_.line_warps = wpb;
-    const int items = h_prefix_[nsys_];
     cfg_.line_grid = std::max(1, std::min((items + wpb - 1) / wpb, sms_ * bpsm));
     // which line kernels the batch needs (systems with no line work count for none)
     // rows per access of the warp kernel: four when every system's lines start on
     // 16-byte boundaries (the mixed form's padded FP32 arrays) and its lanes' spans
     // are multiples of four, two when they start on 8- or 16-byte boundaries
-    cfg_.line_thread = cfg_.line_warp = cfg_.line_single = 0;
+    cfg_.line_thread = cfg_.line_warp = cfg_.line_single = cfg_.line_reg = 0;
     cfg_.line_vw = elem == 4 ? 4 : 2;
     for (int s = 0; s < nsys_; ++s) {
-        if (h_prefix_[s + 1] == h_prefix_[s]) continue;
+        if (h_prefix_[s + 1] == h_prefix_[s] && h_prefix_[lists + s + 1] == h_prefix_[lists + s]) continue;
         const SysDev &d = h_sys_[s];
         if (d.line_kind == LK_THREAD) {
             cfg_.line_thread = 1;
+        } else if (d.line_kind == LK_REG) {
+            cfg_.line_reg |= d.line_np <= 1 ? 1 : 2;
         } else {
             cfg_.line_warp = 1;
             if (d.jp & 1) cfg_.line_single = 1;
@@ -479,15 +475,33 @@ int Engine::configure_lines(int elem, int only_L)
         }
     }
     if (cfg_.line_single) cfg_.line_vw = 1;
-    if (!cfg_.line_thread && !cfg_.line_warp) cfg_.line_warp = 1;  // empty batch: a no-op launch
+    if (!cfg_.line_thread && !cfg_.line_warp && !cfg_.line_reg) cfg_.line_warp = 1;  // empty batch: a no-op launch
+    for (int q = 0; q < 2; ++q) {
+        const int rocc = elem == 4 ? line_reg_occupancy<float>(q + 1) : line_reg_occupancy<double>(q + 1);
+        cfg_.line_grid_reg[q] = std::max(1, std::min((reg_items + 3) / 4, sms_ * rocc));
+    }
     const int tocc = elem == 4 ? line_thread_occupancy<float>() : line_thread_occupancy<double>();
     cfg_.line_grid_thread = std::max(1, std::min((items + 3) / 4, sms_ * tocc));
     return 0;
 }
 
+// Full passes of G row chunks (32 bytes each) over a line of length L in
+// k_jline_reg; half a chunk may follow them.  0 when the kernel does not serve the
+// shape (FP64 lines of odd length, which start on 8-byte boundaries, among them).
+static int reg_passes(int L, int elem, int G)
+{
+    if (G < REG_MIN_LANES || (elem == 8 && (L & 1))) return 0;
+    const int chunk = G * 32 / elem, half = 16 / elem;
+    const int np = std::max(1, (L - half + chunk - 1) / chunk);
+    return np <= REG_PASSES ? np : 0;
+}
+
+// Most rows per lane the autotuner gives the shared-memory kernel, whose staging
+// grows with the batch's largest rows per lane.
 static constexpr int MAX_TUNED_ROWS = 17;
 
-// Rows per lane; one lane per line (G = 1) stages nothing, so it counts as one.
+// Rows per lane of the shared-memory kernel; one lane per line (G = 1) stages
+// nothing, so it counts as one.
 static int rows_for(int L, int G)
 {
     if (G == 1) return 1;
@@ -497,46 +511,54 @@ static int rows_for(int L, int G)
     return c;
 }
 
-static void set_shape(int L, int lanes, int *G, int *c, int *kind)
+// A line shape: lanes per line, plus LINE_STAGED for the shared-memory kernel where
+// the lanes' registers would hold the line too.
+static constexpr int LINE_STAGED = 0x100;
+
+static void set_shape(SysDev &d, int elem, int shape)
 {
-    const int g = std::max(1, std::min(lanes, 32));
-    *G = g;
-    *c = rows_for(L, g);
-    *kind = g == 1 ? LK_THREAD : LK_WARP;
+    const int g = std::max(1, std::min(shape & (LINE_STAGED - 1), 32));
+    d.lane_group = g;
+    d.rows_per_lane = rows_for(d.jmax2, g);
+    d.line_np = (shape & LINE_STAGED) ? 0 : reg_passes(d.jmax2, elem, g);
+    d.line_kind = g == 1 ? LK_THREAD : d.line_np ? LK_REG : LK_WARP;
 }
 
-// Lanes per J-line for a line of length L: a forced value, the autotuner's
-// choice for (precision, L), or the default of line_shape().
-void Engine::shape_for(int L, int elem, int forced, int *G, int *c, int *kind)
+// Lanes per J-line of a system (jmax2 set): a forced value, the autotuner's
+// choice for (precision, line length), or the default: the smallest power of two
+// that leaves at most 12 rows per lane (at most 32 lanes), widened while the
+// lanes' registers cannot hold the line.
+void Engine::shape_for(SysDev &d, int elem, int forced)
 {
     if (forced > 0) {
         int g = 1;
         while (g * 2 <= std::min(forced, 32)) g *= 2;
-        set_shape(L, g, G, c, kind);
+        set_shape(d, elem, g);
         return;
     }
     {
         std::lock_guard<std::mutex> lk(tunes().mu);
-        auto it = tunes().lanes.find(std::make_pair(elem, L));
+        auto it = tunes().lanes.find(std::make_pair(elem, d.jmax2));
         if (it != tunes().lanes.end()) {
-            set_shape(L, it->second, G, c, kind);
+            set_shape(d, elem, it->second);
             return;
         }
     }
-    line_shape(L, G, c);
-    *kind = *G == 1 ? LK_THREAD : LK_WARP;
+    int g = 1;
+    while (g < 32 && g * 12 < d.jmax2) g *= 2;
+    const int np = reg_passes(d.jmax2, elem, 32);
+    while (g > 1 && g < 32 && np && reg_passes(d.jmax2, elem, g) != np) g *= 2;
+    set_shape(d, elem, g);
 }
 
 // The autotuner: for the line lengths of the batch without a recorded choice, time
 // a red/black pass of the J-line kernel over all their lines at once (the other
-// systems' line work masked out) for each lanes-per-line value g, each length
-// taking the smallest power of two at or above g that leaves it at most
-// MAX_TUNED_ROWS rows per lane, and keep the fastest g for all of them.  Timing
-// the whole mix at once ranks the shapes as the batch runs them: timing each
-// length alone, on its few systems, left a 512-system FP64 batch 10% slower than
-// one shape for every line.  The row bound keeps the kernel's shared-memory
-// staging, sized by the batch's largest rows per lane, small enough for full
-// occupancy.
+// systems' line work masked out) for each lanes-per-line value g and each of the
+// two kernels, each length taking the shape nearest to it that can hold its lines
+// (shape_of below), and keep the fastest for all of them.  Timing the whole mix at
+// once ranks the shapes as the batch runs them: timing each length alone, on its
+// few systems, left a 512-system FP64 batch 10% slower than one shape for every
+// line.
 int Engine::autotune_lines(const SolveOptions &opt, int elem)
 {
     std::vector<int> todo;
@@ -561,21 +583,29 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
         w[q].write_old = 1;
         w[q].gate = G_ANY;
     }
-    // lanes of length L under the candidate g: the smallest power of two at or
-    // above g within the row bound; for a line too long for the bound at any
-    // width, 32 while its staging stays within 48 KB per warp, else none (0:
-    // the candidate is skipped; one lane per line always fits)
-    auto lanes_for = [&](int L, int g) {
+    // the shape of length L under the candidate (g, staged): the smallest power of
+    // two at or above g at which k_jline_reg takes its fewest passes, or, staged or for
+    // a line that kernel does not serve, that leaves a lane at most MAX_TUNED_ROWS
+    // rows; for a line too long for that, 32 while its staging stays within 48 KB per
+    // warp, else none (0: the candidate is skipped)
+    auto shape_of = [&](int L, int g, bool staged) {
+        if (g == 1) return 1;
+        const int np = reg_passes(L, elem, 32);  // 0: k_jline_reg does not serve L
         for (int h = g; h <= 32; h *= 2) {
-            int G = 1, c = 1, kind = LK_WARP;
-            set_shape(L, h, &G, &c, &kind);
-            if (kind != LK_WARP || (c <= MAX_TUNED_ROWS && (size_t)kernel_smem_line_bytes(c, elem) <= 48 * 1024))
-                return h;
+            if (np > 0 && !staged) {
+                if (reg_passes(L, elem, h) == np) return h;
+            } else if (rows_for(L, h) <= MAX_TUNED_ROWS &&
+                       (size_t)kernel_smem_line_bytes(rows_for(L, h), elem) <= 48 * 1024) {
+                return np > 0 ? h | LINE_STAGED : h;
+            }
         }
-        int G = 1, c = 1, kind = LK_WARP;
-        set_shape(L, 32, &G, &c, &kind);
-        return (size_t)kernel_smem_line_bytes(c, elem) <= 48 * 1024 ? 32 : 0;
+        return (size_t)kernel_smem_line_bytes(rows_for(L, 32), elem) <= 48 * 1024 ? (np > 0 ? 32 | LINE_STAGED : 32) : 0;
     };
+    bool any_reg = false, any_long = false;
+    for (int L : todo) {
+        any_reg = any_reg || reg_passes(L, elem, 32) > 0;
+        any_long = any_long || L > 32;
+    }
     // the timing events and the tuning mask are released on every way out
     struct TuneScope {
         std::vector<int> &mask;
@@ -592,15 +622,22 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
     const cudaEvent_t e0 = scope.e0, e1 = scope.e1;
     tune_lengths_ = todo;
     int best_g = 0;
+    bool best_staged = false;
     float best_ms = 1e30f;
-    for (int g = 1; g <= 32; g *= 2) {
+    // both kernels at every width (k_jline takes 60.6 us against 66.1 for four FP32
+    // half-sweeps of 145x173x100 cells, 336 against 290 of 258^3); one lane per line
+    // for short lines only (at 66 cells it takes nine times the best width's time)
+    for (int cand = any_long ? 1 : 0; cand < (any_reg ? 12 : 6); ++cand) {
+        const int g = 1 << cand % 6;
+        const bool staged = cand >= 6;
+        if (g == 1 && staged) continue;
         bool fits = true;
-        for (int L : todo) fits = fits && lanes_for(L, g) > 0;
+        for (int L : todo) fits = fits && shape_of(L, g, staged) > 0;
         if (!fits) continue;
         for (int s = 0; s < nsys_; ++s) {
             const int L = h_sys_[s].jmax2;
             if (h_sys_[s].n > 0 && std::find(todo.begin(), todo.end(), L) != todo.end())
-                set_shape(L, lanes_for(L, g), &h_sys_[s].lane_group, &h_sys_[s].rows_per_lane, &h_sys_[s].line_kind);
+                set_shape(h_sys_[s], elem, shape_of(L, g, staged));
         }
         int rc = configure_lines(elem, -1);
         if (rc) return rc;
@@ -615,21 +652,19 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
         if (tot < best_ms) {
             best_ms = tot;
             best_g = g;
+            best_staged = staged;
         }
     }
     for (int L : todo) {
-        int g = best_g > 0 ? lanes_for(L, best_g) : 0;
-        if (g == 0) {  // no candidate timed
-            int c_unused = 0;
-            line_shape(L, &g, &c_unused);
-        }
+        int g = best_g > 0 ? shape_of(L, best_g, best_staged) : 0;
+        if (g == 0) g = L <= 12 ? 1 : 32;  // no candidate timed
         {
             std::lock_guard<std::mutex> lk(tunes().mu);
             tunes().lanes[std::make_pair(elem, L)] = g;
         }
         for (int s = 0; s < nsys_; ++s)
             if (h_sys_[s].jmax2 == L && h_sys_[s].n > 0)
-                set_shape(L, g, &h_sys_[s].lane_group, &h_sys_[s].rows_per_lane, &h_sys_[s].line_kind);
+                set_shape(h_sys_[s], elem, g);
     }
     (void)opt;
     save_tune_cache();
@@ -644,10 +679,12 @@ void Engine::load_tune_cache(const std::string &path)
     if (!f) return;
     int elem, L, G;
     char buf[256];
-    while (std::fgets(buf, sizeof buf, f))
-        if (std::sscanf(buf, " {\"elem\": %d, \"L\": %d, \"lanes\": %d}", &elem, &L, &G) == 3 && G >= 1 &&
-            G <= 32)
-            tunes().lanes[std::make_pair(elem, L)] = G;
+    while (std::fgets(buf, sizeof buf, f)) {
+        int staged = 0;  // absent in files of choices between widths alone
+        if (std::sscanf(buf, " {\"elem\": %d, \"L\": %d, \"lanes\": %d, \"staged\": %d}", &elem, &L, &G, &staged) >= 3 &&
+            G >= 1 && G <= 32)
+            tunes().lanes[std::make_pair(elem, L)] = G | (staged ? LINE_STAGED : 0);
+    }
     std::fclose(f);
 }
 
@@ -661,7 +698,8 @@ void Engine::save_tune_cache()
     std::fprintf(f, "[\n");
     size_t q = 0;
     for (const auto &kv : line_tune_)
-        std::fprintf(f, "  {\"elem\": %d, \"L\": %d, \"lanes\": %d}%s\n", kv.first.first, kv.first.second, kv.second,
+        std::fprintf(f, "  {\"elem\": %d, \"L\": %d, \"lanes\": %d, \"staged\": %d}%s\n", kv.first.first, kv.first.second,
+                     kv.second & (LINE_STAGED - 1), (kv.second & LINE_STAGED) != 0,
                      ++q < line_tune_.size() ? "," : "");
     std::fprintf(f, "]\n");
     std::fclose(f);
@@ -675,7 +713,7 @@ int Engine::tune_table(int *out, int max_entries) const
         if (q < max_entries) {
             out[3 * q] = kv.first.first;
             out[3 * q + 1] = kv.first.second;
-            out[3 * q + 2] = kv.second;
+            out[3 * q + 2] = kv.second & (LINE_STAGED - 1);
         }
         ++q;
     }

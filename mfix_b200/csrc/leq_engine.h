@@ -204,7 +204,7 @@ private:
     int bind_lists();
     int configure_lines(int elem, int only_L = 0);
     std::vector<int> tune_lengths_;  // configure_lines(elem, -1): the line lengths being tuned
-    void shape_for(int L, int elem, int forced, int *G, int *c, int *kind);
+    void shape_for(SysDev &d, int elem, int forced);
     int autotune_lines(const SolveOptions &opt, int elem);
     void save_tune_cache();
 
@@ -358,16 +358,13 @@ private:
 
 SolveResult result_of(const SysState &st, bool mixed);
 
-// choice of lanes per J-line and rows per lane for a line of length L
-void line_shape(int L, int *G, int *c);
-
 // Work memory of one system with n cells and `lines` J-lines: the iteration
 // vectors and factors of the given precision, plus the initial-guess copy of
 // the mixed form (work_bytes); live_work_bytes also leaves room for an FP64
 // re-solve of a mixed attempt in the same block.
 size_t vec_region_bytes(int64_t n, int64_t lines, int precision);
 // Line pitch and cells of the arrays in a form's precision (the mixed form pads
-// each J-line of its FP32 arrays to a multiple of four cells).
+// each J-line of its FP32 arrays to a multiple of eight cells).
 int form_pitch(int jmax2, int precision);
 int64_t form_cells(int64_t n, int64_t lines, int precision);
 size_t work_bytes(int64_t n, int64_t lines, int precision);

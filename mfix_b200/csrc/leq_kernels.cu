@@ -2543,6 +2543,34 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? (VW == 4 ? 5 : 6) : 4) k
     }
 }
 
+// A line on which DGTSV interchanges rows or meets a zero pivot, solved by one
+// thread: the matrix rows in the line's factor cells (unused for a flagged line),
+// INFO first, from the matrix alone, then the solve in the destination.
+template <typename T>
+__device__ __forceinline__ void flagged_line(const SysDev &d, SysState &st, const LineCtx<T> &x, T *dstp, const T *oldl,
+                                             bool write_old)
+{
+    const int L = x.L;
+    T *sub = reinterpret_cast<T *>(d.fac[0]) + x.base;
+    T *dg = reinterpret_cast<T *>(d.fac[1]) + x.base;
+    T *sup = reinterpret_cast<T *>(d.fac[2]) + x.base;
+    T f_unused;
+    for (int r = 0; r < L; ++r) line_row<T>(x, r, sub[r], dg[r], sup[r], f_unused);
+    const int skip = dgtsv_info<T>(L, sub, dg, sup) != 0;
+    atomicAdd(&st.line_fallbacks, 1);
+    if (skip) {
+        atomicAdd(&st.line_skips, 1);
+        if (write_old)
+            for (int r = 0; r < L; ++r) dstp[r] = oldl[r];
+        return;
+    }
+    // the right-hand side of row r goes to the line's own cell r of the
+    // destination; a later row reads only its own cell (a neighbour that
+    // clamps onto itself), so the rows are formed before they are overwritten
+    for (int r = 0; r < L; ++r) line_row<T>(x, r, sub[r], dg[r], sup[r], dstp[r]);
+    dgtsv_rows<T>(L, sub, dg, sup, dstp);
+}
+
 // ------------------------------------------------------------------ J-line half-sweep, one lane per line
 // For short lines in large numbers (batches and serving) each lane runs the two
 // recurrences down its own line, keeping y in the destination (the line's own
@@ -2598,29 +2626,400 @@ __global__ void __launch_bounds__(128) k_jline_thread(BatchView b, WaveArgs w)
                     dstp[r] = xv;
                 }
             } else {
-                // DGTSV with interchanges: the matrix rows in the line's factor cells
-                // (unused for a flagged line); INFO first, from the matrix alone
-                T *sub = reinterpret_cast<T *>(d.fac[0]) + x.base;
-                T *dg = reinterpret_cast<T *>(d.fac[1]) + x.base;
-                T *sup = reinterpret_cast<T *>(d.fac[2]) + x.base;
-                T f_unused;
-                for (int r = 0; r < L; ++r) line_row<T>(x, r, sub[r], dg[r], sup[r], f_unused);
-                const int skip = dgtsv_info<T>(L, sub, dg, sup) != 0;
-                atomicAdd(&st.line_fallbacks, 1);
-                if (skip) {
-                    atomicAdd(&st.line_skips, 1);
-                    const T *oldl = vec<T>(d, w.old) + x.base;
-                    if (w.write_old)
-                        for (int r = 0; r < L; ++r) dstp[r] = oldl[r];
-                } else {
-                    // the right-hand side of row r goes to the line's own cell r of the
-                    // destination; a later row reads only its own cell (a neighbour that
-                    // clamps onto itself), so the rows are formed before they are overwritten
-                    for (int r = 0; r < L; ++r) line_row<T>(x, r, sub[r], dg[r], sup[r], dstp[r]);
-                    dgtsv_rows<T>(L, sub, dg, sup, dstp);
-                }
+                flagged_line<T>(d, st, x, dstp, vec<T>(d, w.old) + x.base, w.write_old);
             }
         }
+    }
+}
+
+// ------------------------------------------------------------------ J-line half-sweep in registers
+// G lanes share a line (32/G lines per warp).  Its rows are taken in chunks of 32
+// bytes (GR rows: eight in FP32, four in FP64); in pass p lane q holds chunk
+// p*G + q, and half a chunk may follow the last full pass (JMAX2 = 2^k + 2 leaves
+// such a remainder), which every lane of the line solves for itself from a copy in
+// shared memory.  All twelve rows of a line are loaded before the first is used
+// and everything else stays in registers: each lane forms its chunk's affine map,
+// one shuffle scan per pass (the passes' scans side by side) composes the maps, and
+// the value at a pass's end carries into the next.
+//
+// A chunk is one 256-bit access in the mixed form's padded arrays, whose lines
+// start on 32-byte boundaries, and two 16-byte accesses in the caller's FP64 arrays
+// with an even JMAX2, which meet again in L1.  (Odd JMAX2, FP64: four 8-byte
+// accesses per chunk took 41.1 us per half-sweep on 129x147x122 cells against 33.8
+// of k_jline, which keeps those lines.)
+//
+// Bound by HBM: 258^3 cells, one half-sweep (20 / 40 bytes per cell): FP32 86.0 us
+// with k_jline's exchange through shared memory (1050 warp instructions a line),
+// 73.2 us here; FP64 153.3 and 143.3 us.  Three blocks of four warps per SM (150
+// registers) keep the rows of twelve lines in flight per SM; four blocks spill and
+// take 302 us for four half-sweeps against 240 of the same loop without spills.
+enum : int { LR_F = 0, LR_L, LR_R, LR_Q, LR_M0, LR_M1, LR_M2, LR_M3, LR_N };  // B, factors, A(-1), A(1), A(-3), A(3)
+
+// A warp's copy of what every line of the system it works on needs.
+struct alignas(16) LineSys {
+    const char *arr[LR_N];  // the rows' arrays
+    const char *nbr, *old;  // neighbour source, own old values
+    char *dst;
+    int64_t c2;             // bytes from a line to the next in K
+    int c1;                 // bytes from a line to the next in I
+    int g0;                 // the system's first work item
+    int lg;                 // log2 of the lanes per line
+    int np;                 // full passes
+    int rows;               // line pitch
+    int extra;              // 1: half a chunk follows the last full pass
+    int imax2, kmax2, do_k, cyc;
+    const int *flags;       // SysDev::line_flag
+};
+
+constexpr int LINE_TAIL = 16 * (32 / REG_MIN_LANES);  // bytes of one row's half chunks past the last pass
+
+// One access (global addresses; the pointers come from memory, so the
+// compiler would use generic ones).
+__device__ __forceinline__ void ld_rows(float *v, const char *p)
+{
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "l"(p));
+}
+__device__ __forceinline__ void ld_rows(double *v, const char *p)
+{
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];\n" : "=d"(v[0]), "=d"(v[1]) : "l"(p));
+}
+__device__ __forceinline__ void st_rows(char *p, const float *v)
+{
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
+                 "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void st_rows(char *p, const double *v)
+{
+    asm volatile("st.global.v2.f64 [%0], {%1, %2};\n" ::"l"(p), "d"(v[0]), "d"(v[1]) : "memory");
+}
+
+template <typename T, int NP>
+__device__ __forceinline__ void reg_line(const BatchView &b, const WaveArgs &wa, const LineSys &c, int sys,
+                                         unsigned char *sm, int i, int k, bool valid)
+{
+    constexpr int GR = 32 / (int)sizeof(T), HR = GR / 2;     // rows of a chunk, of half a chunk
+    constexpr int PC = sizeof(T) == 4 ? 1 : 2, PR = GR / PC;  // accesses of a chunk, rows of an access
+    const int lg = c.lg, G = 1 << lg, np = c.np, do_k = c.do_k, extra = c.extra;
+    const int lane = threadIdx.x & 31, gl = lane & (G - 1);
+    const int64_t line = (int64_t)(i - 1) * c.c1 + (int64_t)(k - 1) * c.c2;
+    auto on = [&](int p) -> bool { return p == 0 || p < np; };  // the pass takes place (np >= 1)
+
+    // the neighbour lines (clamped onto the line itself at the array edge, wrapped
+    // along a cyclic axis)
+    const char *nbr = c.nbr + line, *old = c.old + line, *xim, *xip, *xkm, *xkp;
+    if (!c.cyc) {
+        xim = i > 1 ? nbr - c.c1 : old;
+        xip = i < c.imax2 ? nbr + c.c1 : old;
+        xkm = k > 1 ? nbr - c.c2 : old;
+        xkp = k < c.kmax2 ? nbr + c.c2 : old;
+    } else {
+        const int im = inc_m(i - 1, c.imax2, c.cyc & 1), ip = inc_p(i - 1, c.imax2, c.cyc & 1);
+        const int km = inc_m(k - 1, c.kmax2, c.cyc & 4), kp = inc_p(k - 1, c.kmax2, c.cyc & 4);
+        xim = im ? nbr + im * (int64_t)c.c1 : old;
+        xip = ip ? nbr + ip * (int64_t)c.c1 : old;
+        xkm = km ? nbr + km * c.c2 : old;
+        xkp = kp ? nbr + kp * c.c2 : old;
+    }
+
+    // ---- the rows.  An access past the line reads the line's first rows and is
+    // zeroed below.
+    T y[NP][GR], l[NP][GR], r[NP][GR], q[NP][GR];
+    int off[NP][PC];
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+        for (int h = 0; h < PC; ++h) {
+            const int at = GR * (p * G + gl) + PR * h;
+            off[p][h] = on(p) && at < c.rows ? at * (int)sizeof(T) : 0;
+        }
+    auto row = [&](const char *src, T(&v)[NP][GR]) {
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+            if (on(p))
+#pragma unroll
+                for (int h = 0; h < PC; ++h) ld_rows(&v[p][PR * h], src + off[p][h]);
+    };
+    unsigned char *te = sm + 16 * (lane >> lg);
+    if (extra) {  // the half chunk past the last pass, a row per lane
+        const int64_t past = 32 * G * np;
+        for (int w = gl; w < LR_N + 4; w += G) {
+            if (!do_k && (w & 2) && w > LR_Q) continue;  // A(-3), A(3) and the K neighbours
+            const char *src = w < LR_N ? c.arr[w & (LR_N - 1)] + line
+                              : w == LR_N ? xim : w == LR_N + 1 ? xip : w == LR_N + 2 ? xkm : xkp;
+            cp_async<16>(te + w * LINE_TAIL, src + past, 16);
+        }
+    }
+    {
+        T m0[NP][GR], m1[NP][GR], x0[NP][GR], x1[NP][GR];
+        row(c.arr[LR_F] + line, y);
+        row(c.arr[LR_M0] + line, m0);
+        row(xim, x0);
+        row(c.arr[LR_M1] + line, m1);
+        row(xip, x1);
+        if (do_k) {
+            T m2[NP][GR], m3[NP][GR], x2[NP][GR], x3[NP][GR];
+            row(c.arr[LR_M2] + line, m2);
+            row(xkm, x2);
+            row(c.arr[LR_M3] + line, m3);
+            row(xkp, x3);
+            row(c.arr[LR_L] + line, l);
+            row(c.arr[LR_R] + line, r);
+            row(c.arr[LR_Q] + line, q);
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+                if (on(p))
+#pragma unroll
+                    for (int t = 0; t < GR; ++t) {
+                        T f = fnms(m0[p][t], x0[p][t], y[p][t]);
+                        f = fnms(m1[p][t], x1[p][t], f);
+                        f = fnms(m2[p][t], x2[p][t], f);
+                        y[p][t] = fnms(m3[p][t], x3[p][t], f);
+                    }
+        } else {
+            row(c.arr[LR_L] + line, l);
+            row(c.arr[LR_R] + line, r);
+            row(c.arr[LR_Q] + line, q);
+#pragma unroll
+            for (int p = 0; p < NP; ++p)
+                if (on(p))
+#pragma unroll
+                    for (int t = 0; t < GR; ++t) y[p][t] = fnms(m1[p][t], x1[p][t], fnms(m0[p][t], x0[p][t], y[p][t]));
+        }
+    }
+    const bool flag = valid && c.flags[(i - 1) + (k - 1) * c.imax2] != 0;
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+        if (on(p) && GR * G * (p + 1) > c.rows)
+#pragma unroll
+            for (int t = 0; t < GR; ++t)
+                if (GR * (p * G + gl) + t / PR * PR >= c.rows) y[p][t] = l[p][t] = r[p][t] = q[p][t] = T(0);
+
+    // ---- y_r = f_r - l_r y_{r-1}, on this lane's chunk of each pass
+    T ma[NP], mb[NP];
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+        if (on(p)) {
+            mb[p] = y[p][0];
+            ma[p] = -l[p][0];
+#pragma unroll
+            for (int t = 1; t < GR; ++t) {
+                mb[p] = fnms(l[p][t], mb[p], y[p][t]);
+                ma[p] = -l[p][t] * ma[p];
+            }
+        }
+#pragma unroll
+    for (int dl = 1; dl < 32; dl <<= 1) {
+        if (dl >= G) break;
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+            if (on(p)) {
+                const T pa = __shfl_up_sync(0xffffffffu, ma[p], dl, G), pb = __shfl_up_sync(0xffffffffu, mb[p], dl, G);
+                if (gl >= dl) {
+                    mb[p] = fma_t(ma[p], pb, mb[p]);
+                    ma[p] = mul_t(ma[p], pa);
+                }
+            }
+    }
+    T carry = T(0);
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+        if (on(p)) {
+            const T pb = __shfl_up_sync(0xffffffffu, mb[p], 1, G);
+            T v = gl == 0 ? T(0) : pb;
+            if (p > 0) {
+                const T pa = __shfl_up_sync(0xffffffffu, ma[p], 1, G);
+                v = gl == 0 ? carry : fma_t(pa, carry, pb);
+            }
+            const T eb = __shfl_sync(0xffffffffu, mb[p], G - 1, G);
+            carry = p == 0 ? eb : fma_t(__shfl_sync(0xffffffffu, ma[p], G - 1, G), carry, eb);
+#pragma unroll
+            for (int t = 0; t < GR; ++t) {
+                v = fnms(l[p][t], v, y[p][t]);
+                y[p][t] = v;
+            }
+        }
+
+    // ---- x_r = r_r y_r - q_r x_{r+1}, from the line's end
+    T back = T(0), fe[HR];
+    if (extra) {  // the same in every lane of the line
+        cp_async_wait_all();
+        __syncwarp();
+        auto tail = [&](int w, int t) -> T { return reinterpret_cast<const T *>(te + w * LINE_TAIL)[t]; };
+#pragma unroll
+        for (int t = 0; t < HR; ++t) {
+            T f = fnms(tail(LR_M0, t), tail(LR_N, t), tail(LR_F, t));
+            f = fnms(tail(LR_M1, t), tail(LR_N + 1, t), f);
+            if (do_k) {
+                f = fnms(tail(LR_M2, t), tail(LR_N + 2, t), f);
+                f = fnms(tail(LR_M3, t), tail(LR_N + 3, t), f);
+            }
+            carry = fnms(tail(LR_L, t), carry, f);
+            fe[t] = carry;
+        }
+#pragma unroll
+        for (int t = HR - 1; t >= 0; --t) {
+            back = fnms(tail(LR_Q, t), back, mul_t(tail(LR_R, t), fe[t]));
+            fe[t] = back;
+        }
+        __syncwarp();  // the next line's copies come after these reads
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+        if (on(p)) {
+#pragma unroll
+            for (int t = 0; t < GR; ++t) y[p][t] = mul_t(r[p][t], y[p][t]);
+            mb[p] = y[p][GR - 1];
+            ma[p] = -q[p][GR - 1];
+#pragma unroll
+            for (int t = GR - 2; t >= 0; --t) {
+                mb[p] = fnms(q[p][t], mb[p], y[p][t]);
+                ma[p] = -q[p][t] * ma[p];
+            }
+        }
+#pragma unroll
+    for (int dl = 1; dl < 32; dl <<= 1) {
+        if (dl >= G) break;
+#pragma unroll
+        for (int p = 0; p < NP; ++p)
+            if (on(p)) {
+                const T na = __shfl_down_sync(0xffffffffu, ma[p], dl, G),
+                        nb = __shfl_down_sync(0xffffffffu, mb[p], dl, G);
+                if (gl + dl < G) {
+                    mb[p] = fma_t(ma[p], nb, mb[p]);
+                    ma[p] = mul_t(ma[p], na);
+                }
+            }
+    }
+#pragma unroll
+    for (int p = NP - 1; p >= 0; --p)
+        if (on(p)) {
+            const T na = __shfl_down_sync(0xffffffffu, ma[p], 1, G), nb = __shfl_down_sync(0xffffffffu, mb[p], 1, G);
+            T v = gl == G - 1 ? back : fma_t(na, back, nb);
+            if (p > 0)
+                back = fma_t(__shfl_sync(0xffffffffu, ma[p], 0, G), back, __shfl_sync(0xffffffffu, mb[p], 0, G));
+#pragma unroll
+            for (int t = GR - 1; t >= 0; --t) {
+                v = fnms(q[p][t], v, y[p][t]);
+                y[p][t] = v;
+            }
+        }
+
+    if (!valid) return;
+    char *dst = c.dst + line;
+    if (flag) {  // DGTSV interchanges rows or meets a zero pivot
+        if (gl == 0) {
+            const SysDev &d = b.sys[sys];
+            LineCtx<T> x;
+            x.a = diag_base<T>(d);
+            x.rhs = vec<T>(d, wa.rhs);
+            x.n = cells<T>(d);
+            x.L = d.jmax2;
+            x.do_k = do_k;
+            x.base = line / (int64_t)sizeof(T);
+            x.nb_im = reinterpret_cast<const T *>(xim);
+            x.nb_ip = reinterpret_cast<const T *>(xip);
+            x.nb_km = reinterpret_cast<const T *>(xkm);
+            x.nb_kp = reinterpret_cast<const T *>(xkp);
+            flagged_line<T>(d, b.st[sys], x, reinterpret_cast<T *>(dst), reinterpret_cast<const T *>(old), wa.write_old);
+        }
+        return;
+    }
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+        if (on(p))
+#pragma unroll
+            for (int h = 0; h < PC; ++h)
+                if (GR * (p * G + gl) + PR * h < c.rows) st_rows(dst + off[p][h], &y[p][PR * h]);
+    if (extra && gl < HR && GR * G * np + gl < c.rows) {  // a row per lane
+        T v = fe[0];
+#pragma unroll
+        for (int t = 1; t < HR; ++t)
+            if (gl == t) v = fe[t];
+        reinterpret_cast<T *>(dst + 32 * G * np)[gl] = v;
+    }
+}
+
+// NP: passes over a line at most (SysDev::line_np).
+template <typename T, int NP>
+__global__ void __launch_bounds__(128, NP == 1 ? 3 : 2) k_jline_reg(const BatchView b, const WaveArgs w)
+{
+    __shared__ LineSys s_sys[4];
+    __shared__ __align__(16) unsigned char s_tail[4][(LR_N + 4) * LINE_TAIL];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    LineSys &c = s_sys[warp];
+    const int total = w.kind == 0 ? b.reg_prefix[b.nsys] : w.count;
+    const bool many = w.kind == 0 && b.nsys > 1;
+    // a warp takes `run` consecutive items at a time: in a batch they mostly belong to
+    // one system, whose fields it then reads once (64 systems of 18-98 cells per line,
+    // four half-sweeps: 274 us with 1, 231 with 2, 223 with 4)
+    const int warps = gridDim.x * 4, run = !many ? 1 : total >= 8 * warps ? 4 : total >= 4 * warps ? 2 : 1;
+    auto sys_of = [&](int item) -> int { return many && item < total ? __ldg(b.reg_sys + item) : 0; };
+    int cur = -1;
+    bool take = false;
+    int item = (blockIdx.x * 4 + warp) * run, left = run, sys = sys_of(item), after;
+    for (; item < total; item = after) {
+        after = item + 1;
+        if (--left == 0) {
+            after += (warps - 1) * run;
+            left = run;
+        }
+        const int next = sys_of(after);  // loaded while this item is processed
+        if (sys != cur) {
+            cur = sys;
+            const SysDev &d = b.sys[sys];
+            take = gate_ok(b.st[sys], w.gate) && d.line_kind == LK_REG && (d.line_np <= 1) == (NP == 1);
+            __syncwarp();
+            if (lane < LR_N) {
+                const int dg = lane == LR_M0 ? 2 : lane == LR_M1 ? 4 : lane == LR_M2 ? 0 : 6;
+                const T *arr = lane == LR_F   ? vec<T>(d, w.rhs)
+                               : lane < LR_M0 ? reinterpret_cast<const T *>(d.fac[lane - LR_L])
+                                              : diag_base<T>(d) + (int64_t)dg * cells<T>(d);
+                c.arr[lane] = reinterpret_cast<const char *>(arr);
+            }
+            if (lane == LR_N) {
+                const int G = d.lane_group, rows = pitch<T>(d);
+                c.nbr = reinterpret_cast<const char *>(vec<T>(d, w.nbr));
+                c.old = reinterpret_cast<const char *>(vec<T>(d, w.old));
+                c.dst = reinterpret_cast<char *>(vec<T>(d, w.dst));
+                c.c1 = rows * (int)sizeof(T);
+                c.c2 = (int64_t)c.c1 * d.imax2;
+                c.g0 = w.kind == 0 ? b.reg_prefix[sys] : 0;
+                c.lg = 31 - __clz(G);
+                c.np = d.line_np;
+                c.rows = rows;
+                c.extra = 32 / (int)sizeof(T) * G * d.line_np < d.jmax2;
+                c.imax2 = d.imax2;
+                c.kmax2 = d.kmax2;
+                c.do_k = d.do_k;
+                c.cyc = d.cyc;
+                c.flags = d.line_flag;
+            }
+            __syncwarp();
+        }
+        if (take) {
+            const int slot = ((item - c.g0) << (5 - c.lg)) + (lane >> c.lg);
+            int i, k;
+            bool valid;
+            if (w.kind == 0) {
+                valid = wave_line(b.sys[sys], w, slot, i, k);
+            } else if (w.kind == 1) {
+                const int ilo = max(1, w.par - c.kmax2);
+                i = ilo + slot;
+                k = w.par - i;
+                valid = i <= min(c.imax2, w.par - 1);
+            } else {
+                valid = slot < w.nlines;
+                const int2 lk = valid ? w.list[slot] : make_int2(1, 1);
+                i = lk.x;
+                k = lk.y;
+            }
+            if (!valid) i = k = 1;  // reads line (1, 1) and stores nothing
+            reg_line<T, NP>(b, w, c, sys, s_tail[warp], i, k, valid);
+        }
+        sys = next;
     }
 }
 
@@ -3244,6 +3643,24 @@ int line_thread_occupancy()
     return nb > 0 ? nb : 1;
 }
 
+template <typename K>
+static int occ(K kern, int threads = CELL_THREADS)
+{
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, threads, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return 2;
+    }
+    return nb > 0 ? nb : 1;
+}
+
+template <typename T>
+int line_reg_occupancy(int np)
+{
+    static const int nb[2] = {occ(k_jline_reg<T, 1>, 128), occ(k_jline_reg<T, REG_PASSES>, 128)};
+    return nb[np <= 1 ? 0 : 1];
+}
+
 // Resident blocks per SM of the staged matvec (shared memory above the default
 // limit is requested first); 0 when it cannot run.
 template <int CFG>
@@ -3283,17 +3700,6 @@ static void launch_staged(const BatchView &b, const LaunchCfg &c, int src)
     }
 }
 
-template <typename K>
-static int occ(K kern)
-{
-    int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, CELL_THREADS, 0) != cudaSuccess) {
-        cudaGetLastError();
-        return 2;
-    }
-    return nb > 0 ? nb : 1;
-}
-
 // Resident blocks per SM of each cell kernel (persistent grids).
 void cell_occupancy(bool fp32, CellOcc *o)
 {
@@ -3321,9 +3727,12 @@ void cell_occupancy(bool fp32, CellOcc *o)
 template <typename T>
 cudaError_t launch_jline(const BatchView &b, const LaunchCfg &c, const WaveArgs &w)
 {
-    // systems with one lane per line, then those with several: one warp-kernel
-    // launch, the two-row instance when all their lines have even length
+    // systems with one lane per line, those whose lines fit their lanes' registers,
+    // and the longer ones: one warp-kernel launch, the two-row instance when all
+    // their lines have even length
     if (c.line_thread) k_jline_thread<T><<<c.line_grid_thread, 128, 0, c.stream>>>(b, w);
+    if (c.line_reg & 1) k_jline_reg<T, 1><<<c.line_grid_reg[0], 128, 0, c.stream>>>(b, w);
+    if (c.line_reg & 2) k_jline_reg<T, REG_PASSES><<<c.line_grid_reg[1], 128, 0, c.stream>>>(b, w);
     if (c.line_warp) {
         const int smem = c.line_warps * kernel_smem_line_bytes(c.line_cmax, (int)sizeof(T));
         constexpr int VMAX = sizeof(T) == 4 ? 4 : 2;
@@ -3452,6 +3861,7 @@ cudaError_t launch_seq_lines(const BatchView &b, const SeqLineArgs &a, cudaStrea
                                                 cudaStream_t, int);                                       \
     template cudaError_t launch_seq_lines<T>(const BatchView &, const SeqLineArgs &, cudaStream_t);        \
     template int prepare_line_kernel<T>(int, int *);                                                     \
+    template int line_reg_occupancy<T>(int);                                                             \
     template int line_thread_occupancy<T>();                                                             \
     template cudaError_t launch_line_factor<T>(const BatchView &, const LaunchCfg &, const int *, int);
 #define INST_TM(T, M)                                                                       \

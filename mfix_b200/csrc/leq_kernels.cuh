@@ -11,8 +11,10 @@ struct BatchView {
     const Tile *tiles;     // [ntiles]
     int ntiles;
     int nsys;
-    const int *line_prefix;  // [nsys+1] parity-wave work items (exclusive prefix)
-    const int *line_sys;     // [items] the system of each parity-wave work item
+    const int *line_prefix;  // [nsys+1] parity-wave work items of k_jline / k_jline_thread (exclusive prefix)
+    const int *line_sys;     // [items] the system of each of them
+    const int *reg_prefix;   // the same of k_jline_reg
+    const int *reg_sys;
     double *partials;        // [ntiles_total * 2]
 };
 
@@ -31,7 +33,10 @@ struct LaunchCfg {
     int line_warps;  // warps per block of the J-line kernel
     int line_grid_thread;  // blocks of the one-lane-per-line kernel (4 warps each)
     int line_thread;       // 1: some system has one lane per line
-    int line_warp;         // 1: some system has several lanes per line
+    int line_warp;         // 1: some system has several lanes per line, its rows in shared memory
+    int line_reg;          // some system has several lanes per line, its rows in their registers: 1 in one pass,
+                           // 2 in more
+    int line_grid_reg[2];  // blocks of those kernels (4 warps each)
     int line_single;       // 1: some system with several lanes per line has an odd line pitch
     int line_vw;           // rows per access of the warp J-line kernel (1, 2 or 4)
     cudaStream_t stream;
@@ -120,6 +125,8 @@ cudaError_t launch_seq_lines(const BatchView &b, const SeqLineArgs &a, cudaStrea
 int kernel_smem_line_bytes(int cmax, int elem_bytes);
 template <typename T>
 int prepare_line_kernel(int cmax, int *warps);
+template <typename T>
+int line_reg_occupancy(int np);  // resident blocks per SM of k_jline_reg for lines of up to np passes
 template <typename T>
 int line_thread_occupancy();  // resident blocks per SM of the one-lane-per-line kernel
 //  // sets the smem attribute, returns resident blocks per SM

@@ -154,7 +154,7 @@ int Engine::live_add(const LiveSystem &ls)
     d.div_jp = make_fastdiv((uint32_t)d.jp);
     d.pc = live_opt_.pc;
     d.ntiles = (int)((std::max(sp.n, d.np) + TILE_CELLS - 1) / TILE_CELLS);
-    shape_for(sp.jmax2, mixed ? 4 : 8, live_opt_.force_lanes, &d.lane_group, &d.rows_per_lane, &d.line_kind);
+    shape_for(d, mixed ? 4 : 8, live_opt_.force_lanes);
     d.half_lines = (sp.imax2 + 1) / 2;
     d.div_h = make_fastdiv((uint32_t)d.half_lines);
     d.a64 = sp.a;

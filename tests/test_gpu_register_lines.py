@@ -1,0 +1,63 @@
+"""J-line kernels around the edges of their shapes: chunk remainders, one and two
+passes, widths that leave lanes idle, short and long lines, both precisions.
+
+Each line is solved by LEQ_MSOLVE (model/leqsol_mod.f:286-598) through the GPU
+and through the oracle; the recurrences are re-associated, so the results differ
+by a few roundings of a diagonally dominant solve: 1e-12 in FP64.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from mfix_b200 import leq
+from mfix_b200 import systems as S
+
+pytestmark = pytest.mark.gpu
+
+
+# interior J cells: L = J + 2; FP64 chunks are 4 rows, half chunks 2, FP32's 8 and 4
+@pytest.mark.parametrize("jmax", [1, 2, 5, 6, 14, 16, 17, 30, 62, 64, 66, 126, 128, 130, 254, 256, 258, 300])
+def test_msolve_line_lengths(cuda, jmax):
+    s = S.conv_diff(5, jmax, 4, seed=jmax)
+    dev = "cuda"
+    a, b = cuda.from_numpy(s.a).to(dev), cuda.from_numpy(s.b).to(dev)
+    x = cuda.zeros(s.n, dtype=cuda.float64, device=dev)
+    cuda.cuda.synchronize()
+    g = leq.geom(s.imax2, s.jmax2, s.kmax2, s.do_k)
+    assert leq.leq_msolve(g, b.data_ptr(), a.data_ptr(), x.data_ptr(), "RSRS", "LINE") == 0
+    want = oracle.msolve(s, s.b)[1]
+    got = x.cpu().numpy()
+    assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("jmax", [6, 30, 34, 62, 66, 126, 130, 254, 258, 262, 300])
+@pytest.mark.parametrize("lanes", [4, 8, 16, 32])
+def test_solve_line_lengths(cuda, precision, jmax, lanes):
+    """Whole solves with a forced width: the true residual meets TOL, the mixed form without a hand-over."""
+    s = S.conv_diff(6, jmax, 5, seed=jmax, tol=1e-8)
+    w = s.copy()
+    assert leq.set_option("line_lanes", lanes) == 0 and leq.set_option("precision", precision) == 0
+    try:
+        assert leq.solve_system(w) == 0
+        assert leq.last_stats()["fp64_fallback"] == 0
+    finally:
+        leq.set_option("precision", 0)
+        leq.set_option("line_lanes", 0)
+    r = w.b - S.matvec_np(w.imax2, w.jmax2, w.kmax2, w.do_k, w.a, w.x)
+    assert np.linalg.norm(r) <= 1.01e-8 * np.linalg.norm(w.b)
+
+
+def test_batch_of_mixed_parities_equals_alone(cuda):
+    """FP64 systems of even and odd JMAX2 in one batch (two line kernels): each as alone."""
+    sysm = [S.conv_diff(9, j, 7, seed=j) for j in (20, 21, 62, 63, 128, 131, 10)]
+    alone = []
+    for s in sysm:
+        w = s.copy()
+        assert leq.solve_system(w) == 0
+        alone.append(w)
+    batch = [s.copy() for s in sysm]
+    rc, res = leq.batch_solve(batch)
+    assert rc == 0
+    for w, v, r in zip(alone, batch, res):
+        assert r.ier == 0 and np.array_equal(w.x, v.x)
