@@ -178,7 +178,9 @@ const char *mfixgpu_last_error(void);
  *   "rtilde_seed"    seed of the Rtilde random stream (replaces RANDOM_NUMBER, model/leq_bicgs.f:298)
  *   "inner_tol"      mixed form: drop of the FP32 residual between FP64 reliable updates (default 1e-2)
  *   "check_every"    iterations between host polls of convergence (default 4)
- *   "use_graph"      1 (default) replay the iteration body as a CUDA graph
+ *   "use_graph"      1 (default) replay the iteration body as a CUDA graph, or run the iterations of a
+ *                    small batch (at most one cell tile per SM) in one cooperative launch; 0: launch
+ *                    every kernel by itself (the same bits)
  *   "time_kernels"   1: time every J-line sweep launch with CUDA events (no graph replay)
  *   "autotune"       1 (default): lanes per J-line picked by measurement for the new line lengths of a
  *                    solve or batch (one lanes-per-line value timed on all their lines at once)

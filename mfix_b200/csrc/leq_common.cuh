@@ -190,6 +190,31 @@ struct WaveArgs {
     int lvl;         // kind 0: 0 every line of the parity, else only lines of wrap level lvl - 1
 };
 
+// Arrivals of k_iterate's barrier of one system, kept on the device between launches.
+struct GroupBar {
+    unsigned count;  // blocks that have arrived, all barriers of the running launch
+    unsigned pad0[31];
+    unsigned left;   // blocks that have left the launch
+    unsigned pad1[31];
+};
+
+// One block of k_iterate: its system, its number among the system's blocks (blocks
+// below the system's tile count own that tile) and their count.
+struct IterBlock {
+    int sys, idx, count, pad;
+};
+
+// One launch of k_iterate.
+struct IterArgs {
+    const IterBlock *blocks;
+    int nblocks;
+    int iterations;  // at most
+    int ns;          // half-sweeps per LEQ_MSOLVE
+    int line_warp, line_cmax;  // as in LaunchCfg
+    GroupBar *bar;   // [nsys]
+    unsigned *abort; // a wait ran out of time
+};
+
 enum Gate : int {
     G_INNER = 0,        // running, inner phase
     G_INNER_NOSNORM = 1,// running, inner phase, no Snorm exit this iteration

@@ -104,6 +104,8 @@ Engine::~Engine()
     cudaFree(d_partials_);
     cudaFree(d_lines_);
     cudaFree(d_seq_scratch_);
+    cudaFree(d_bar_);
+    cudaFree(d_iter_blocks_);
     cudaFree(d_one_sys_);
     cudaFree(d_dot_partials_);
     cudaFree(gm_basis_);
@@ -364,7 +366,7 @@ int Engine::setup_batch(const std::vector<SystemSpec> &specs, const SolveOptions
     CK(upload(&d_st_, &st_cap_, h_st_.data(), h_st_.size(), stream_));
     CK(upload(&d_tiles_, &tiles_cap_, h_tiles_.data(), h_tiles_.size(), stream_));
     CK(upload(&d_allprefix_, &allprefix_cap_, h_allprefix_.data(), h_allprefix_.size(), stream_));
-    const size_t need_part = 2 * (size_t)std::max(tile_base, 1);
+    const size_t need_part = 4 * (size_t)std::max(tile_base, 1);  // two sets of partial sums
     if (need_part > part_cap_) {
         cudaFree(d_partials_);
         d_partials_ = nullptr;
@@ -624,13 +626,16 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
     int best_g = 0;
     bool best_staged = false;
     float best_ms = 1e30f;
-    // both kernels at every width (k_jline takes 60.6 us against 66.1 for four FP32
-    // half-sweeps of 145x173x100 cells, 336 against 290 of 258^3); one lane per line
-    // for short lines only (at 66 cells it takes nine times the best width's time)
-    for (int cand = any_long ? 1 : 0; cand < (any_reg ? 12 : 6); ++cand) {
-        const int g = 1 << cand % 6;
-        const bool staged = cand >= 6;
-        if (g == 1 && staged) continue;
+    // the register kernel's one shape first (the fewest lanes that hold a line in its
+    // fewest passes: more lanes idle), then k_jline at every width, which has to be 5%
+    // faster where the register kernel serves the batch (60.6 us against 66.1 for four
+    // FP32 half-sweeps of 145x173x100 cells, 336 against 290 of 258^3): k_iterate, which
+    // has few warps, prefers the shape with the most lines a warp.  One lane per line
+    // for short lines only (at 66 cells it takes nine times the best width's time).
+    for (int cand = any_reg ? -1 : any_long ? 1 : 0; cand < 6; ++cand) {
+        if (any_reg && cand == 0) continue;
+        const int g = cand < 0 ? 2 : 1 << cand;
+        const bool staged = cand > 0 && any_reg;
         bool fits = true;
         for (int L : todo) fits = fits && shape_of(L, g, staged) > 0;
         if (!fits) continue;
@@ -649,7 +654,7 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
         CK(cudaEventRecord(e1, stream_));
         CK(cudaEventSynchronize(e1));
         cudaEventElapsedTime(&tot, e0, e1);
-        if (tot < best_ms) {
+        if (tot < (staged && !best_staged ? 0.95f : 1.f) * best_ms) {
             best_ms = tot;
             best_g = g;
             best_staged = staged;
@@ -1312,6 +1317,78 @@ int Engine::launch_body(const SolveOptions &opt)
     return 0;
 }
 
+// Whether the batch's iterations run as k_iterate: BiCGSTAB with red/black sweeps, no
+// line of more than one pass, and a block per cell tile that are all resident (one per
+// SM); larger batches need the launches' own grids, with more warps per SM.
+bool Engine::small_batch(const SolveOptions &opt, IterArgs *a)
+{
+    if (!opt.use_graph || opt.time_kernels || opt.method != 2 || opt.pc != PC_LINE) return false;
+    if (cfg_.line_thread || (cfg_.line_reg & 2) || view_.ntiles < 1 || view_.ntiles > sms_) return false;
+    for (int q = 0; q < 2; ++q) {
+        if (plan_[q].empty() || plan_[q].size() != plan_[0].size()) return false;
+        for (const Step &st : plan_[q])
+            if (st.type != 0 || st.w.kind != 0 || st.w.lvl != 0) return false;
+    }
+    *a = IterArgs{};
+    a->ns = (int)plan_[0].size();
+    a->line_warp = cfg_.line_warp;
+    a->line_cmax = cfg_.line_cmax;
+    if (!(opt.precision == PREC_MIXED ? iterate_fits<float, true>(*a) : iterate_fits<double, false>(*a))) return false;
+    if ((size_t)nsys_ + 1 > bar_cap_) {
+        cudaFree(d_bar_);
+        d_bar_ = nullptr;
+        bar_cap_ = 0;
+        bar_dirty_ = true;
+        if (cudaMalloc((void **)&d_bar_, sizeof(GroupBar) * ((size_t)nsys_ + 1)) != cudaSuccess) {
+            cudaGetLastError();
+            d_bar_ = nullptr;
+            return false;
+        }
+        bar_cap_ = (size_t)nsys_ + 1;
+    }
+    // a block per tile; the SMs left over go to the systems whose lines need more
+    // rounds of a block's eight warps than one, in proportion to what they miss
+    h_iter_blocks_.clear();
+    const int lists = nsys_ + 1, spare = sms_ - view_.ntiles;
+    auto missing = [&](int s) {
+        const int q = h_sys_[s].line_kind == LK_REG ? lists : 0;
+        return std::max(0, (h_prefix_[q + s + 1] - h_prefix_[q + s] + 7) / 8 - h_sys_[s].ntiles);
+    };
+    auto used = [&](int s) { return h_sys_[s].n > 0; };  // not an empty slot of a live batch
+    int64_t all = 0;
+    for (int s = 0; s < nsys_; ++s) all += used(s) ? missing(s) : 0;
+    for (int s = 0; s < nsys_; ++s) {
+        if (!used(s)) continue;
+        const int more = all > spare ? (int)(missing(s) * (int64_t)spare / all) : missing(s);
+        const int count = h_sys_[s].ntiles + more;
+        for (int q = 0; q < count; ++q) h_iter_blocks_.push_back(IterBlock{s, q, count, 0});
+    }
+    a->nblocks = (int)h_iter_blocks_.size();
+    if (stage_open(sizeof(IterBlock) * h_iter_blocks_.size() + 256) != cudaSuccess ||
+        upload_staged(&d_iter_blocks_, &iter_blocks_cap_, h_iter_blocks_.data(), h_iter_blocks_.size()) != cudaSuccess ||
+        stage_close() != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    a->blocks = d_iter_blocks_;
+    a->bar = d_bar_ + 1;
+    a->abort = &d_bar_->count;
+    return true;
+}
+
+cudaError_t Engine::run_iterations(const SolveOptions &opt, IterArgs a, int iterations)
+{
+    if (bar_dirty_) {
+        const cudaError_t e = cudaMemsetAsync(d_bar_, 0, sizeof(GroupBar) * bar_cap_, stream_);
+        if (e != cudaSuccess) return e;
+        bar_dirty_ = false;
+    }
+    a.iterations = iterations;
+    ++launches_;
+    return opt.precision == PREC_MIXED ? launch_iterate<float, true>(view_, cfg_, a)
+                                       : launch_iterate<double, false>(view_, cfg_, a);
+}
+
 // One batch whose arrays are all on the device.
 int Engine::run_batch(const std::vector<SystemSpec> &specs, const SolveOptions &opt, std::vector<SolveResult> &out)
 {
@@ -1362,7 +1439,9 @@ int Engine::run_batch(const std::vector<SystemSpec> &specs, const SolveOptions &
     int max_itmax = 0;
     for (const auto &s : specs) max_itmax = std::max(max_itmax, s.itmax);
     const int max_loops = std::max(1, max_itmax + 2);
-    const bool graph = opt.use_graph && !ktime_;
+    IterArgs iter{};
+    const bool small = small_batch(opt, &iter);
+    const bool graph = opt.use_graph && !ktime_ && !small;
     cudaGraphExec_t gexec = nullptr;
     long long per_body = 0;
     if (graph) {
@@ -1398,7 +1477,22 @@ int Engine::run_batch(const std::vector<SystemSpec> &specs, const SolveOptions &
     const int K = ktime_ ? 1 : std::max(1, opt.check_every);
     int loops = 0, snap = 0;
     bool have_prev = false, finished = false;
-    while (loops < max_loops && !finished) {
+    // k_iterate returns when every system is done: one launch, as a rule
+    constexpr int SMALL_CHUNK = 256;
+    for (; small && loops < max_loops && !finished; loops += SMALL_CHUNK) {
+        CK(run_iterations(opt, iter, std::min(SMALL_CHUNK, max_loops - loops)));
+        CK(launch_state_snapshot(d_st_, d_st_mapped_, nsys_, stream_));
+        ++launches_;
+        CK(cudaEventRecord(ev_a_, stream_));
+        CK(cudaEventSynchronize(ev_a_));
+        finished = true;
+        for (int s = 0; s < nsys_; ++s) {
+            const SysState &st = h_st_pinned_[s];
+            finished = finished && (st.status != ST_RUNNING || (st.err & 4));
+            bar_dirty_ = bar_dirty_ || (st.err & 4);
+        }
+    }
+    while (!small && loops < max_loops && !finished) {
         for (int q = 0; q < K && loops < max_loops; ++q, ++loops)
             if ((rc = run_once())) {
                 if (gexec) cudaGraphExecDestroy(gexec);

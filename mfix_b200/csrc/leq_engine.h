@@ -312,6 +312,17 @@ private:
     };
     std::vector<ListRef> list_refs_;
 
+    // small batches: whole iterations in one cooperative launch (k_iterate)
+    GroupBar *d_bar_ = nullptr;  // one per system, then the abort word
+    size_t bar_cap_ = 0;
+    bool bar_dirty_ = true;      // they have to be cleared before the next launch
+    std::vector<IterBlock> h_iter_blocks_;
+    IterBlock *d_iter_blocks_ = nullptr;
+    size_t iter_blocks_cap_ = 0;
+    bool live_small_ = false;
+    bool small_batch(const SolveOptions &opt, IterArgs *a);
+    cudaError_t run_iterations(const SolveOptions &opt, IterArgs a, int iterations);
+
     // standalone kernels
     SysDev *d_one_sys_ = nullptr;
     double *d_dot_partials_ = nullptr;
@@ -339,6 +350,7 @@ private:
     int live_commit();
     int live_take(long long q, std::vector<LiveDone> &done);
     SolveOptions live_opt_{};
+    IterArgs live_iter_{};
     std::vector<char> slot_used_, slot_fresh_, slot_reported_, slot_cleared_;
     std::vector<LiveSystem> slot_sys_;
     std::vector<long long> slot_join_snap_, slot_join_body_;

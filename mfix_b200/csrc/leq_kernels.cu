@@ -629,6 +629,13 @@ __device__ __forceinline__ float dterm(float acc, float a, float xn, float xc)
 }
 __device__ __forceinline__ float dcentre(float acc, float rowsum, float xc) { return __fmaf_rn(rowsum, xc, acc); }
 
+// The plain form's terms, likewise: the first product rounded, the others fused
+// (which of two products a compiler fuses depends on the code around them).
+__device__ __forceinline__ double term0(double a, double x) { return __dmul_rn(a, x); }
+__device__ __forceinline__ float term0(float a, float x) { return __fmul_rn(a, x); }
+__device__ __forceinline__ double term(double acc, double a, double x) { return __fma_rn(a, x, acc); }
+__device__ __forceinline__ float term(float acc, float a, float x) { return __fmaf_rn(a, x, acc); }
+
 template <typename T, bool DEFECT = false>
 __device__ __forceinline__ T dot_row7(const Row7<T> &r, bool do_k)
 {
@@ -645,14 +652,14 @@ __device__ __forceinline__ T dot_row7(const Row7<T> &r, bool do_k)
         }
         return v;
     }
-    T v = r.a[0] * r.x[0];
-    v = v + r.a[1] * r.x[1];
-    v = v + r.a[2] * r.x[2];
-    v = v + r.a[3] * r.x[3];
-    v = v + r.a[4] * r.x[4];
+    T v = term0(r.a[0], r.x[0]);
+    v = term(v, r.a[1], r.x[1]);
+    v = term(v, r.a[2], r.x[2]);
+    v = term(v, r.a[3], r.x[3]);
+    v = term(v, r.a[4], r.x[4]);
     if (do_k) {
-        v = v + r.a[5] * r.x[5];
-        v = v + r.a[6] * r.x[6];
+        v = term(v, r.a[5], r.x[5]);
+        v = term(v, r.a[6], r.x[6]);
     }
     return v;
 }
@@ -771,21 +778,19 @@ __device__ __forceinline__ vec2_t<T> dot_pair7(const Pair7<T> &r, bool do_k)
         }
         return mk2<T>(u, w);
     }
-    T u = r.a[0].x * r.x[0].x;
-    T w = r.a[0].y * r.x[0].y;
-    u = u + r.a[1].x * r.x[1].x;
-    w = w + r.a[1].y * r.x[1].y;
-    u = u + r.a[2].x * r.x[2].x;
-    w = w + r.a[2].y * r.x[2].y;
-    u = u + r.a[3].x * r.x[3].x;
-    w = w + r.a[3].y * r.x[3].y;
-    u = u + r.a[4].x * r.x[4].x;
-    w = w + r.a[4].y * r.x[4].y;
+    T u = term0(r.a[0].x, r.x[0].x);
+    T w = term0(r.a[0].y, r.x[0].y);
+#pragma unroll
+    for (int q = 1; q < 5; ++q) {
+        u = term(u, r.a[q].x, r.x[q].x);
+        w = term(w, r.a[q].y, r.x[q].y);
+    }
     if (do_k) {
-        u = u + r.a[5].x * r.x[5].x;
-        w = w + r.a[5].y * r.x[5].y;
-        u = u + r.a[6].x * r.x[6].x;
-        w = w + r.a[6].y * r.x[6].y;
+#pragma unroll
+        for (int q = 5; q < 7; ++q) {
+            u = term(u, r.a[q].x, r.x[q].x);
+            w = term(w, r.a[q].y, r.x[q].y);
+        }
     }
     return mk2<T>(u, w);
 }
@@ -804,79 +809,107 @@ __device__ __forceinline__ double zdot2(const unsigned char *z, int64_t c, const
     return (zz.x ? (double)v.x : 0.0) + (zz.y ? (double)v.y : 0.0);
 }
 
+// Scalar steps of the kernels below, from the sums over a system's cells.
+__device__ inline void fin_p(SysState &s, const double (&tot)[1]) { s.defl_cp = tot[0] / s.defl_e; }
+__device__ inline void fin_alpha(SysState &s, const double (&tot)[1]) { s.alpha = s.rho / tot[0]; }
+template <bool MIXED>
+__device__ inline void fin_s(SysState &s, const double (&tot)[MIXED ? 2 : 1])
+{
+    s.snorm = sqrt(tot[0]);
+    if (MIXED)
+        s.snorm_exit = (s.snorm <= 0.1 * s.tol * s.outer_rnorm0) ? 1 : 0;
+    else
+        s.snorm_exit = (!s.icheck && s.snorm <= DBL_EPSILON) ? 1 : 0;  // TOLMIN = EPSILON(ONE); none with
+                                                                      // MINIMIZE_DOTPRODUCTS
+    if (MIXED && s.defl) s.defl_cs = tot[MIXED ? 1 : 0] / s.defl_e;
+}
+__device__ inline void fin_omega(SysState &s, const double (&tot)[2])
+{
+    double txt = tot[1];
+    if (txt == 0.0) txt = 1.0e-15;  // SMALL_NUMBER
+    s.omega = tot[0] / txt;
+}
+
 // P = R (i = 1) or P = R + beta*(P - omega*V) (model/leq_bicgs.f:334-343).
 // Deflated mixed systems also form c_p = z^T P / z^T A z.
+// One tile of it, U2 cell pairs per thread and pass; true when zv holds a sum.
+template <typename T, bool MIXED, int U2>
+__device__ __forceinline__ bool p_tile(const SysDev &d, const SysState &st, int idx, double (&zv)[1])
+{
+    const int64_t c0 = (int64_t)idx * TILE_CELLS;
+    const int cnt = (int)min((int64_t)TILE_CELLS, cells<T>(d) - c0);
+    const T *__restrict__ r = vec<T>(d, V_R) + c0;
+    T *__restrict__ p = vec<T>(d, V_P) + c0;
+    const int np = cnt >> 1;  // cell pairs; an odd last cell is done by thread 0
+    const bool defl = MIXED && st.defl;
+    if (st.i == 1) {
+        for (int base = threadIdx.x; base < np; base += U2 * blockDim.x) {
+            vec2_t<T> rv[U2];
+#pragma unroll
+            for (int u = 0; u < U2; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) rv[u] = ld2(r + 2 * q);
+            }
+#pragma unroll
+            for (int u = 0; u < U2; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    st2(p + 2 * q, rv[u]);
+                    if (defl) zv[0] += zdot2<T>(d.defl_z, c0 + 2 * q, rv[u]);
+                }
+            }
+        }
+        if ((cnt & 1) && threadIdx.x == 0) {
+            p[cnt - 1] = r[cnt - 1];
+            if (defl && d.defl_z[c0 + cnt - 1]) zv[0] += (double)r[cnt - 1];
+        }
+    } else {
+        const T beta = (T)st.beta, omega = (T)st.omega;
+        const T *__restrict__ v = vec<T>(d, V_V) + c0;
+        for (int base = threadIdx.x; base < np; base += U2 * blockDim.x) {
+            vec2_t<T> rv[U2], pv[U2], vv[U2];
+#pragma unroll
+            for (int u = 0; u < U2; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    rv[u] = ld2(r + 2 * q);
+                    pv[u] = ld2(p + 2 * q);
+                    vv[u] = ld2(v + 2 * q);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U2; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    const vec2_t<T> pn = mk2<T>(rv[u].x + beta * (pv[u].x - omega * vv[u].x),
+                                                rv[u].y + beta * (pv[u].y - omega * vv[u].y));
+                    st2(p + 2 * q, pn);
+                    if (defl) zv[0] += zdot2<T>(d.defl_z, c0 + 2 * q, pn);
+                }
+            }
+        }
+        if ((cnt & 1) && threadIdx.x == 0) {
+            const int c = cnt - 1;
+            p[c] = r[c] + beta * (p[c] - omega * v[c]);
+            if (defl && d.defl_z[c0 + c]) zv[0] += (double)p[c];
+        }
+    }
+    return defl;
+}
+
 template <typename T, bool MIXED>
 __global__ void __launch_bounds__(256, 4) k_p_update(BatchView b)
 {
     constexpr int U2 = Batch<T>::STREAM / 2;
     TileRun run{-1, 0};
-    auto fin = [&](SysState &st, const double(&tot)[1]) { st.defl_cp = tot[0] / st.defl_e; };
+    auto fin = [&](SysState &st, const double(&tot)[1]) { fin_p(st, tot); };
     for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
         const Tile tl = b.tiles[t];
         const SysDev &d = b.sys[tl.sys];
         const SysState &st = b.st[tl.sys];
         if (!gate_ok(st, G_INNER)) continue;
-        const int64_t c0 = (int64_t)tl.idx * TILE_CELLS;
-        const int cnt = (int)min((int64_t)TILE_CELLS, cells<T>(d) - c0);
-        const T *__restrict__ r = vec<T>(d, V_R) + c0;
-        T *__restrict__ p = vec<T>(d, V_P) + c0;
-        const int np = cnt >> 1;  // cell pairs; an odd last cell is done by thread 0
-        const bool defl = MIXED && st.defl;
         double zv[1] = {0.0};
-        if (st.i == 1) {
-            for (int base = threadIdx.x; base < np; base += U2 * blockDim.x) {
-                vec2_t<T> rv[U2];
-#pragma unroll
-                for (int u = 0; u < U2; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) rv[u] = ld2(r + 2 * q);
-                }
-#pragma unroll
-                for (int u = 0; u < U2; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        st2(p + 2 * q, rv[u]);
-                        if (defl) zv[0] += zdot2<T>(d.defl_z, c0 + 2 * q, rv[u]);
-                    }
-                }
-            }
-            if ((cnt & 1) && threadIdx.x == 0) {
-                p[cnt - 1] = r[cnt - 1];
-                if (defl && d.defl_z[c0 + cnt - 1]) zv[0] += (double)r[cnt - 1];
-            }
-        } else {
-            const T beta = (T)st.beta, omega = (T)st.omega;
-            const T *__restrict__ v = vec<T>(d, V_V) + c0;
-            for (int base = threadIdx.x; base < np; base += U2 * blockDim.x) {
-                vec2_t<T> rv[U2], pv[U2], vv[U2];
-#pragma unroll
-                for (int u = 0; u < U2; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        rv[u] = ld2(r + 2 * q);
-                        pv[u] = ld2(p + 2 * q);
-                        vv[u] = ld2(v + 2 * q);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U2; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        const vec2_t<T> pn = mk2<T>(rv[u].x + beta * (pv[u].x - omega * vv[u].x),
-                                                    rv[u].y + beta * (pv[u].y - omega * vv[u].y));
-                        st2(p + 2 * q, pn);
-                        if (defl) zv[0] += zdot2<T>(d.defl_z, c0 + 2 * q, pn);
-                    }
-                }
-            }
-            if ((cnt & 1) && threadIdx.x == 0) {
-                const int c = cnt - 1;
-                p[c] = r[c] + beta * (p[c] - omega * v[c]);
-                if (defl && d.defl_z[c0 + c]) zv[0] += (double)p[c];
-            }
-        }
-        if (defl) {
+        if (p_tile<T, MIXED, U2>(d, st, tl.idx, zv)) {
             tile_partial<1>(b, d, tl.idx, zv);
             run_add<1>(b, run, tl.sys, fin);
         }
@@ -946,86 +979,92 @@ __global__ void __launch_bounds__(256, 4) k_copy(BatchView b, int src, int dst, 
 }
 
 // V = A*Phat and alpha = rho / (Rtilde, V) (model/leq_bicgs.f:355-361).
+// One tile of it: U one-cell rows or UP cell pairs per thread and pass.
+template <typename T, bool MIXED, bool PAIR, int U, int UP>
+__device__ __forceinline__ void alpha_tile(const SysDev &d, const SysState &st, int src, int idx, double (&v)[1])
+{
+    const int64_t c0 = (int64_t)idx * TILE_CELLS;
+    const int cnt = (int)min((int64_t)TILE_CELLS, cells<T>(d) - c0);
+    const T *__restrict__ a = diag_base<T>(d);
+    const T *__restrict__ x = vec<T>(d, src);
+    const T *__restrict__ rt = vec<T>(d, V_RT);
+    T *__restrict__ y = vec<T>(d, V_V);
+    // deflated mixed systems: V = A (Phat + c_p z) = A Phat + c_p A z
+    const bool defl = MIXED && st.defl;
+    const double cp = defl ? st.defl_cp : 0.0;
+    if constexpr (PAIR) {
+        const int np = cnt >> 1;
+        for (int base = threadIdx.x; base < np; base += UP * blockDim.x) {
+            Pair7<T> rw[UP];
+            int jr[UP];
+            vec2_t<T> rtv[UP];
+#pragma unroll
+            for (int u = 0; u < UP; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    load_pair7<T, MIXED>(d, a, x, c0 + 2 * q, rw[u], &jr[u]);
+                    rtv[u] = ld2(rt + c0 + 2 * q);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < UP; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    vec2_t<T> yv = dot_pair7<T, MIXED>(rw[u], d.do_k);
+                    if (jr[u] >= d.jmax2) yv.x = T(0);  // pad cells of the padded FP32 arrays
+                    if (jr[u] + 1 >= d.jmax2) yv.y = T(0);
+                    if (defl) {
+                        const float2 az = ld2(d.defl_az + c0 + 2 * q);
+                        yv.x = yv.x + (T)(cp * (double)az.x);
+                        yv.y = yv.y + (T)(cp * (double)az.y);
+                    }
+                    st2(y + c0 + 2 * q, yv);
+                    v[0] += (double)rtv[u].x * (double)yv.x;
+                    v[0] += (double)rtv[u].y * (double)yv.y;
+                }
+            }
+        }
+    } else {
+    for (int base = threadIdx.x; base < cnt; base += U * blockDim.x) {
+        Row7<T> rw[U];
+        int jr[U];
+        T rtv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = base + u * blockDim.x;
+            if (c < cnt) {
+                load_row7<T, T, MIXED>(d, a, x, c0 + c, rw[u], &jr[u]);
+                rtv[u] = rt[c0 + c];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = base + u * blockDim.x;
+            if (c < cnt) {
+                T yv = dot_row7<T, MIXED>(rw[u], d.do_k);
+                if (jr[u] >= d.jmax2) yv = T(0);
+                if (defl) yv = yv + (T)(cp * (double)d.defl_az[c0 + c]);
+                y[c0 + c] = yv;
+                v[0] += (double)rtv[u] * (double)yv;
+            }
+        }
+    }
+    }
+}
+
 template <typename T, bool MIXED, bool PAIR>
 __global__ void __launch_bounds__(256) k_matvec_alpha(BatchView b, int src)
 {
-    constexpr int U = 2;  // one-cell rows: two cells per thread and pass (80 registers in FP32)
-    constexpr int UP = 1;  // one cell pair per thread and pass: fewer registers, more resident warps
     TileRun run{-1, 0};
-    auto fin = [&](SysState &st, const double(&tot)[1]) { st.alpha = st.rho / tot[0]; };
+    auto fin = [&](SysState &st, const double(&tot)[1]) { fin_alpha(st, tot); };
     for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
         const Tile tl = b.tiles[t];
         const SysDev &d = b.sys[tl.sys];
         SysState &st = b.st[tl.sys];
         if (!gate_ok(st, G_INNER) || pair_rows<T>(d) != PAIR) continue;
-        const int64_t c0 = (int64_t)tl.idx * TILE_CELLS;
-        const int cnt = (int)min((int64_t)TILE_CELLS, cells<T>(d) - c0);
-        const T *__restrict__ a = diag_base<T>(d);
-        const T *__restrict__ x = vec<T>(d, src);
-        const T *__restrict__ rt = vec<T>(d, V_RT);
-        T *__restrict__ y = vec<T>(d, V_V);
         double v[1] = {0.0};
-        // deflated mixed systems: V = A (Phat + c_p z) = A Phat + c_p A z
-        const bool defl = MIXED && st.defl;
-        const double cp = defl ? st.defl_cp : 0.0;
-        if constexpr (PAIR) {
-            const int np = cnt >> 1;
-            for (int base = threadIdx.x; base < np; base += UP * blockDim.x) {
-                Pair7<T> rw[UP];
-                int jr[UP];
-                vec2_t<T> rtv[UP];
-#pragma unroll
-                for (int u = 0; u < UP; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        load_pair7<T, MIXED>(d, a, x, c0 + 2 * q, rw[u], &jr[u]);
-                        rtv[u] = ld2(rt + c0 + 2 * q);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < UP; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        vec2_t<T> yv = dot_pair7<T, MIXED>(rw[u], d.do_k);
-                        if (jr[u] >= d.jmax2) yv.x = T(0);  // pad cells of the padded FP32 arrays
-                        if (jr[u] + 1 >= d.jmax2) yv.y = T(0);
-                        if (defl) {
-                            const float2 az = ld2(d.defl_az + c0 + 2 * q);
-                            yv.x = yv.x + (T)(cp * (double)az.x);
-                            yv.y = yv.y + (T)(cp * (double)az.y);
-                        }
-                        st2(y + c0 + 2 * q, yv);
-                        v[0] += (double)rtv[u].x * (double)yv.x;
-                        v[0] += (double)rtv[u].y * (double)yv.y;
-                    }
-                }
-            }
-        } else {
-        for (int base = threadIdx.x; base < cnt; base += U * blockDim.x) {
-            Row7<T> rw[U];
-            int jr[U];
-            T rtv[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int c = base + u * blockDim.x;
-                if (c < cnt) {
-                    load_row7<T, T, MIXED>(d, a, x, c0 + c, rw[u], &jr[u]);
-                    rtv[u] = rt[c0 + c];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int c = base + u * blockDim.x;
-                if (c < cnt) {
-                    T yv = dot_row7<T, MIXED>(rw[u], d.do_k);
-                    if (jr[u] >= d.jmax2) yv = T(0);
-                    if (defl) yv = yv + (T)(cp * (double)d.defl_az[c0 + c]);
-                    y[c0 + c] = yv;
-                    v[0] += (double)rtv[u] * (double)yv;
-                }
-            }
-        }
-        }
+        // one pair: fewer registers, more resident warps; two one-cell rows: 80 registers in FP32
+        alpha_tile<T, MIXED, PAIR, 2, 1>(d, st, src, tl.idx, v);
         tile_partial<1>(b, d, tl.idx, v);
         run_add<1>(b, run, tl.sys, fin);
     }
@@ -1034,66 +1073,65 @@ __global__ void __launch_bounds__(256) k_matvec_alpha(BatchView b, int src)
 
 // S = R - alpha*V and Snorm (model/leq_bicgs.f:365-375); deflated mixed systems
 // also form c_s = z^T S / z^T A z.
+// One tile of it, U2 cell pairs per thread and pass.
+template <typename T, bool MIXED, int U2, int NV = MIXED ? 2 : 1>
+__device__ __forceinline__ void s_tile(const SysDev &d, const SysState &st, int idx, double (&v)[NV])
+{
+    const int64_t c0 = (int64_t)idx * TILE_CELLS;
+    const int cnt = (int)min((int64_t)TILE_CELLS, cells<T>(d) - c0);
+    const T alpha = (T)st.alpha;
+    const T *__restrict__ r = vec<T>(d, V_R) + c0;
+    const T *__restrict__ vv = vec<T>(d, V_V) + c0;
+    T *__restrict__ s = vec<T>(d, V_S) + c0;
+    const bool defl = MIXED && st.defl;
+    const int np = cnt >> 1;
+    for (int base = threadIdx.x; base < np; base += U2 * blockDim.x) {
+        vec2_t<T> rv[U2], wv[U2];
+#pragma unroll
+        for (int u = 0; u < U2; ++u) {
+            const int q = base + u * blockDim.x;
+            if (q < np) {
+                rv[u] = ld2(r + 2 * q);
+                wv[u] = ld2(vv + 2 * q);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U2; ++u) {
+            const int q = base + u * blockDim.x;
+            if (q < np) {
+                const T s0 = rv[u].x - alpha * wv[u].x, s1 = rv[u].y - alpha * wv[u].y;
+                st2(s + 2 * q, mk2<T>(s0, s1));
+                v[0] += (double)s0 * (double)s0;
+                v[0] += (double)s1 * (double)s1;
+                if (defl) v[NV - 1] += zdot2<T>(d.defl_z, c0 + 2 * q, mk2<T>(s0, s1));
+            }
+        }
+    }
+    if ((cnt & 1) && threadIdx.x == 0) {
+        const int c = cnt - 1;
+        const T sv = r[c] - alpha * vv[c];
+        s[c] = sv;
+        v[0] += (double)sv * (double)sv;
+        if (defl && d.defl_z[c0 + c]) v[NV - 1] += (double)sv;
+    }
+}
+
 template <typename T, bool MIXED>
 __global__ void __launch_bounds__(256, 4) k_s_update(BatchView b)
 {
     constexpr int U2 = Batch<T>::STREAM / 2;
     constexpr int NV = MIXED ? 2 : 1;
     TileRun run{-1, 0};
-    auto fin = [&](SysState &st, const double(&tot)[NV]) {
-        st.snorm = sqrt(tot[0]);
-        if (MIXED)
-            st.snorm_exit = (st.snorm <= 0.1 * st.tol * st.outer_rnorm0) ? 1 : 0;
-        else
-            st.snorm_exit = (!st.icheck && st.snorm <= DBL_EPSILON) ? 1 : 0;  // TOLMIN = EPSILON(ONE); none
-                                                                              // with MINIMIZE_DOTPRODUCTS
-        if (MIXED && st.defl) st.defl_cs = tot[NV - 1] / st.defl_e;
-    };
+    auto fin = [&](SysState &st, const double(&tot)[NV]) { fin_s<MIXED>(st, tot); };
     for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
         const Tile tl = b.tiles[t];
         const SysDev &d = b.sys[tl.sys];
         SysState &st = b.st[tl.sys];
         if (!gate_ok(st, G_INNER)) continue;
-        const int64_t c0 = (int64_t)tl.idx * TILE_CELLS;
-        const int cnt = (int)min((int64_t)TILE_CELLS, cells<T>(d) - c0);
-        const T alpha = (T)st.alpha;
-        const T *__restrict__ r = vec<T>(d, V_R) + c0;
-        const T *__restrict__ vv = vec<T>(d, V_V) + c0;
-        T *__restrict__ s = vec<T>(d, V_S) + c0;
-        const bool defl = MIXED && st.defl;
         double v[NV];
 #pragma unroll
         for (int k = 0; k < NV; ++k) v[k] = 0.0;
-        const int np = cnt >> 1;
-        for (int base = threadIdx.x; base < np; base += U2 * blockDim.x) {
-            vec2_t<T> rv[U2], wv[U2];
-#pragma unroll
-            for (int u = 0; u < U2; ++u) {
-                const int q = base + u * blockDim.x;
-                if (q < np) {
-                    rv[u] = ld2(r + 2 * q);
-                    wv[u] = ld2(vv + 2 * q);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U2; ++u) {
-                const int q = base + u * blockDim.x;
-                if (q < np) {
-                    const T s0 = rv[u].x - alpha * wv[u].x, s1 = rv[u].y - alpha * wv[u].y;
-                    st2(s + 2 * q, mk2<T>(s0, s1));
-                    v[0] += (double)s0 * (double)s0;
-                    v[0] += (double)s1 * (double)s1;
-                    if (defl) v[NV - 1] += zdot2<T>(d.defl_z, c0 + 2 * q, mk2<T>(s0, s1));
-                }
-            }
-        }
-        if ((cnt & 1) && threadIdx.x == 0) {
-            const int c = cnt - 1;
-            const T sv = r[c] - alpha * vv[c];
-            s[c] = sv;
-            v[0] += (double)sv * (double)sv;
-            if (defl && d.defl_z[c0 + c]) v[NV - 1] += (double)sv;
-        }
+        s_tile<T, MIXED, U2>(d, st, tl.idx, v);
         tile_partial<NV>(b, d, tl.idx, v);
         run_add<NV>(b, run, tl.sys, fin);
     }
@@ -1101,93 +1139,95 @@ __global__ void __launch_bounds__(256, 4) k_s_update(BatchView b)
 }
 
 // T = A*Shat, omega = (T,S)/(T,T) with (T,T) = 0 -> SMALL_NUMBER (model/leq_bicgs.f:409-427).
+// One tile of it: U one-cell rows or UP cell pairs per thread and pass.
+template <typename T, bool MIXED, bool PAIR, int U, int UP>
+__device__ __forceinline__ void omega_tile(const SysDev &d, const SysState &st, int src, int idx, double (&v)[2])
+{
+    const int64_t c0 = (int64_t)idx * TILE_CELLS;
+    const int cnt = (int)min((int64_t)TILE_CELLS, cells<T>(d) - c0);
+    const T *__restrict__ a = diag_base<T>(d);
+    const T *__restrict__ x = vec<T>(d, src);
+    const T *__restrict__ s = vec<T>(d, V_S);
+    T *__restrict__ y = vec<T>(d, V_T);
+    // deflated mixed systems: T = A (Shat + c_s z) = A Shat + c_s A z
+    const bool defl = MIXED && st.defl;
+    const double cs = defl ? st.defl_cs : 0.0;
+    if constexpr (PAIR) {
+        const int np = cnt >> 1;
+        for (int base = threadIdx.x; base < np; base += UP * blockDim.x) {
+            Pair7<T> rw[UP];
+            int jr[UP];
+            vec2_t<T> sv[UP];
+#pragma unroll
+            for (int u = 0; u < UP; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    load_pair7<T, MIXED>(d, a, x, c0 + 2 * q, rw[u], &jr[u]);
+                    sv[u] = ld2(s + c0 + 2 * q);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < UP; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    vec2_t<T> yv = dot_pair7<T, MIXED>(rw[u], d.do_k);
+                    if (jr[u] >= d.jmax2) yv.x = T(0);  // pad cells of the padded FP32 arrays
+                    if (jr[u] + 1 >= d.jmax2) yv.y = T(0);
+                    if (defl) {
+                        const float2 az = ld2(d.defl_az + c0 + 2 * q);
+                        yv.x = yv.x + (T)(cs * (double)az.x);
+                        yv.y = yv.y + (T)(cs * (double)az.y);
+                    }
+                    st2(y + c0 + 2 * q, yv);
+                    v[0] += (double)yv.x * (double)sv[u].x;
+                    v[1] += (double)yv.x * (double)yv.x;
+                    v[0] += (double)yv.y * (double)sv[u].y;
+                    v[1] += (double)yv.y * (double)yv.y;
+                }
+            }
+        }
+    } else {
+    for (int base = threadIdx.x; base < cnt; base += U * blockDim.x) {
+        Row7<T> rw[U];
+        int jr[U];
+        T sv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = base + u * blockDim.x;
+            if (c < cnt) {
+                load_row7<T, T, MIXED>(d, a, x, c0 + c, rw[u], &jr[u]);
+                sv[u] = s[c0 + c];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = base + u * blockDim.x;
+            if (c < cnt) {
+                T yv = dot_row7<T, MIXED>(rw[u], d.do_k);
+                if (jr[u] >= d.jmax2) yv = T(0);
+                if (defl) yv = yv + (T)(cs * (double)d.defl_az[c0 + c]);
+                y[c0 + c] = yv;
+                v[0] += (double)yv * (double)sv[u];
+                v[1] += (double)yv * (double)yv;
+            }
+        }
+    }
+    }
+}
+
 template <typename T, bool MIXED, bool PAIR>
 __global__ void __launch_bounds__(256) k_matvec_omega(BatchView b, int src)
 {
-    constexpr int U = 2;  // one-cell rows: two cells per thread and pass (80 registers in FP32)
-    constexpr int UP = 1;  // one cell pair per thread and pass: fewer registers, more resident warps
     TileRun run{-1, 0};
-    auto fin = [&](SysState &st, const double(&tot)[2]) {
-        double txt = tot[1];
-        if (txt == 0.0) txt = 1.0e-15;  // SMALL_NUMBER
-        st.omega = tot[0] / txt;
-    };
+    auto fin = [&](SysState &st, const double(&tot)[2]) { fin_omega(st, tot); };
     for (int t = blockIdx.x; t < b.ntiles; t += gridDim.x) {
         const Tile tl = b.tiles[t];
         const SysDev &d = b.sys[tl.sys];
         SysState &st = b.st[tl.sys];
         if (!gate_ok(st, G_INNER_NOSNORM) || pair_rows<T>(d) != PAIR) continue;
-        const int64_t c0 = (int64_t)tl.idx * TILE_CELLS;
-        const int cnt = (int)min((int64_t)TILE_CELLS, cells<T>(d) - c0);
-        const T *__restrict__ a = diag_base<T>(d);
-        const T *__restrict__ x = vec<T>(d, src);
-        const T *__restrict__ s = vec<T>(d, V_S);
-        T *__restrict__ y = vec<T>(d, V_T);
         double v[2] = {0.0, 0.0};
-        // deflated mixed systems: T = A (Shat + c_s z) = A Shat + c_s A z
-        const bool defl = MIXED && st.defl;
-        const double cs = defl ? st.defl_cs : 0.0;
-        if constexpr (PAIR) {
-            const int np = cnt >> 1;
-            for (int base = threadIdx.x; base < np; base += UP * blockDim.x) {
-                Pair7<T> rw[UP];
-                int jr[UP];
-                vec2_t<T> sv[UP];
-#pragma unroll
-                for (int u = 0; u < UP; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        load_pair7<T, MIXED>(d, a, x, c0 + 2 * q, rw[u], &jr[u]);
-                        sv[u] = ld2(s + c0 + 2 * q);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < UP; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        vec2_t<T> yv = dot_pair7<T, MIXED>(rw[u], d.do_k);
-                        if (jr[u] >= d.jmax2) yv.x = T(0);  // pad cells of the padded FP32 arrays
-                        if (jr[u] + 1 >= d.jmax2) yv.y = T(0);
-                        if (defl) {
-                            const float2 az = ld2(d.defl_az + c0 + 2 * q);
-                            yv.x = yv.x + (T)(cs * (double)az.x);
-                            yv.y = yv.y + (T)(cs * (double)az.y);
-                        }
-                        st2(y + c0 + 2 * q, yv);
-                        v[0] += (double)yv.x * (double)sv[u].x;
-                        v[1] += (double)yv.x * (double)yv.x;
-                        v[0] += (double)yv.y * (double)sv[u].y;
-                        v[1] += (double)yv.y * (double)yv.y;
-                    }
-                }
-            }
-        } else {
-        for (int base = threadIdx.x; base < cnt; base += U * blockDim.x) {
-            Row7<T> rw[U];
-            int jr[U];
-            T sv[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int c = base + u * blockDim.x;
-                if (c < cnt) {
-                    load_row7<T, T, MIXED>(d, a, x, c0 + c, rw[u], &jr[u]);
-                    sv[u] = s[c0 + c];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int c = base + u * blockDim.x;
-                if (c < cnt) {
-                    T yv = dot_row7<T, MIXED>(rw[u], d.do_k);
-                    if (jr[u] >= d.jmax2) yv = T(0);
-                    if (defl) yv = yv + (T)(cs * (double)d.defl_az[c0 + c]);
-                    y[c0 + c] = yv;
-                    v[0] += (double)yv * (double)sv[u];
-                    v[1] += (double)yv * (double)yv;
-                }
-            }
-        }
-        }
+        // one pair: fewer registers, more resident warps; two one-cell rows: 80 registers in FP32
+        omega_tile<T, MIXED, PAIR, 2, 1>(d, st, src, tl.idx, v);
         tile_partial<2>(b, d, tl.idx, v);
         run_add<2>(b, run, tl.sys, fin);
     }
@@ -1692,6 +1732,126 @@ __device__ __forceinline__ NatPair nat_pair(const SysDev &d, int64_t p)
     return NatPair{(int64_t)line * d.jmax2 + j, j < d.jmax2, j + 1 < d.jmax2};
 }
 
+// One tile of it, U2 cell pairs per thread and pass.
+template <typename T, bool MIXED, int U2>
+__device__ __forceinline__ void xr_tile(const SysDev &d, const SysState &st, int ph_id, int sh_id, int idx, double (&v)[2])
+{
+    const int64_t c0 = (int64_t)idx * TILE_CELLS;
+    const int cnt = (int)min((int64_t)TILE_CELLS, cells<T>(d) - c0);
+    // FP64 drop-in: X is VAR.  Mixed form: the solution is accumulated in FP64
+    // every iteration (x64 += alpha*Phat + omega*Shat with FP64 scalars), in
+    // VAR's own layout (nat_pair maps the padded pairs onto it).
+    using X_T = typename std::conditional<MIXED, double, T>::type;
+    X_T *__restrict__ x =
+        MIXED ? reinterpret_cast<X_T *>(d.x64[0]) : reinterpret_cast<X_T *>(vec<T>(d, V_X)) + c0;
+    auto xload = [&](int q) -> vec2_t<X_T> {
+        if constexpr (MIXED) {
+            const NatPair np2 = nat_pair(d, c0 + 2 * q);
+            return mk2<X_T>(np2.r0 ? x[np2.c] : X_T(0), np2.r1 ? x[np2.c + 1] : X_T(0));
+        } else {
+            return ld2(x + 2 * q);
+        }
+    };
+    auto xstore = [&](int q, const vec2_t<X_T> &v) {
+        if constexpr (MIXED) {
+            const NatPair np2 = nat_pair(d, c0 + 2 * q);
+            if (np2.r0) x[np2.c] = v.x;
+            if (np2.r1) x[np2.c + 1] = v.y;
+        } else {
+            st2(x + 2 * q, v);
+        }
+    };
+    const X_T alpha = (X_T)st.alpha;
+    const T *__restrict__ ph = vec<T>(d, ph_id) + c0;
+    const int np = cnt >> 1;
+    // deflated mixed systems: Phat + c_p z and Shat + c_s z, so x also gains
+    // (alpha c_p + omega c_s) on the coupled rows
+    const bool defl = MIXED && st.defl;
+    const unsigned char *__restrict__ zr = defl ? d.defl_z + c0 : nullptr;
+    if (st.snorm_exit) {
+        const X_T wz = defl ? (X_T)(st.alpha * st.defl_cp) : X_T(0);
+        for (int base = threadIdx.x; base < np; base += U2 * blockDim.x) {
+            vec2_t<X_T> xv[U2];
+            vec2_t<T> pv[U2];
+#pragma unroll
+            for (int u = 0; u < U2; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    xv[u] = xload(q);
+                    pv[u] = ld2(ph + 2 * q);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U2; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    vec2_t<X_T> xn = mk2<X_T>(xv[u].x + alpha * (X_T)pv[u].x, xv[u].y + alpha * (X_T)pv[u].y);
+                    if (defl) {
+                        const uchar2 zz = *reinterpret_cast<const uchar2 *>(zr + 2 * q);
+                        if (zz.x) xn.x = xn.x + wz;
+                        if (zz.y) xn.y = xn.y + wz;
+                    }
+                    xstore(q, xn);
+                }
+            }
+        }
+        if (!MIXED && (cnt & 1) && threadIdx.x == 0) x[cnt - 1] = x[cnt - 1] + alpha * (X_T)ph[cnt - 1];
+    } else {
+        const X_T omega = (X_T)st.omega;
+        const X_T wz = defl ? (X_T)(st.alpha * st.defl_cp + st.omega * st.defl_cs) : X_T(0);
+        const T omega_t = (T)st.omega;
+        const T *__restrict__ sh = vec<T>(d, sh_id) + c0;
+        const T *__restrict__ s = vec<T>(d, V_S) + c0;
+        const T *__restrict__ tv = vec<T>(d, V_T) + c0;
+        const T *__restrict__ rt = vec<T>(d, V_RT) + c0;
+        T *__restrict__ r = vec<T>(d, V_R) + c0;
+        for (int base = threadIdx.x; base < np; base += U2 * blockDim.x) {
+            vec2_t<X_T> xv[U2];
+            vec2_t<T> pv[U2], hv[U2], sv[U2], tw[U2], rtv[U2];
+#pragma unroll
+            for (int u = 0; u < U2; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    xv[u] = xload(q);
+                    pv[u] = ld2(ph + 2 * q);
+                    hv[u] = ld2(sh + 2 * q);
+                    sv[u] = ld2(s + 2 * q);
+                    tw[u] = ld2(tv + 2 * q);
+                    rtv[u] = ld2(rt + 2 * q);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U2; ++u) {
+                const int q = base + u * blockDim.x;
+                if (q < np) {
+                    vec2_t<X_T> xn = mk2<X_T>(xv[u].x + alpha * (X_T)pv[u].x + omega * (X_T)hv[u].x,
+                                              xv[u].y + alpha * (X_T)pv[u].y + omega * (X_T)hv[u].y);
+                    if (defl) {
+                        const uchar2 zz = *reinterpret_cast<const uchar2 *>(zr + 2 * q);
+                        if (zz.x) xn.x = xn.x + wz;
+                        if (zz.y) xn.y = xn.y + wz;
+                    }
+                    xstore(q, xn);
+                    const T r0 = sv[u].x - omega_t * tw[u].x, r1 = sv[u].y - omega_t * tw[u].y;
+                    st2(r + 2 * q, mk2<T>(r0, r1));
+                    v[0] += (double)r0 * (double)r0;
+                    v[1] += (double)rtv[u].x * (double)r0;
+                    v[0] += (double)r1 * (double)r1;
+                    v[1] += (double)rtv[u].y * (double)r1;
+                }
+            }
+        }
+        if (!MIXED && (cnt & 1) && threadIdx.x == 0) {
+            const int c = cnt - 1;
+            x[c] = x[c] + alpha * (X_T)ph[c] + omega * (X_T)sh[c];
+            const T rv = s[c] - omega_t * tv[c];
+            r[c] = rv;
+            v[0] += (double)rv * (double)rv;
+            v[1] += (double)rt[c] * (double)rv;
+        }
+    }
+}
+
 template <typename T, bool MIXED>
 __global__ void __launch_bounds__(256) k_xr_update(BatchView b, int ph_id, int sh_id)
 {
@@ -1708,121 +1868,8 @@ __global__ void __launch_bounds__(256) k_xr_update(BatchView b, int ph_id, int s
         const SysDev &d = b.sys[tl.sys];
         SysState &st = b.st[tl.sys];
         if (!gate_ok(st, G_INNER)) continue;
-        const int64_t c0 = (int64_t)tl.idx * TILE_CELLS;
-        const int cnt = (int)min((int64_t)TILE_CELLS, cells<T>(d) - c0);
-        // FP64 drop-in: X is VAR.  Mixed form: the solution is accumulated in FP64
-        // every iteration (x64 += alpha*Phat + omega*Shat with FP64 scalars), in
-        // VAR's own layout (nat_pair maps the padded pairs onto it).
-        using X_T = typename std::conditional<MIXED, double, T>::type;
-        X_T *__restrict__ x =
-            MIXED ? reinterpret_cast<X_T *>(d.x64[0]) : reinterpret_cast<X_T *>(vec<T>(d, V_X)) + c0;
-        auto xload = [&](int q) -> vec2_t<X_T> {
-            if constexpr (MIXED) {
-                const NatPair np2 = nat_pair(d, c0 + 2 * q);
-                return mk2<X_T>(np2.r0 ? x[np2.c] : X_T(0), np2.r1 ? x[np2.c + 1] : X_T(0));
-            } else {
-                return ld2(x + 2 * q);
-            }
-        };
-        auto xstore = [&](int q, const vec2_t<X_T> &v) {
-            if constexpr (MIXED) {
-                const NatPair np2 = nat_pair(d, c0 + 2 * q);
-                if (np2.r0) x[np2.c] = v.x;
-                if (np2.r1) x[np2.c + 1] = v.y;
-            } else {
-                st2(x + 2 * q, v);
-            }
-        };
-        const X_T alpha = (X_T)st.alpha;
-        const T *__restrict__ ph = vec<T>(d, ph_id) + c0;
         double v[2] = {0.0, 0.0};
-        const int np = cnt >> 1;
-        // deflated mixed systems: Phat + c_p z and Shat + c_s z, so x also gains
-        // (alpha c_p + omega c_s) on the coupled rows
-        const bool defl = MIXED && st.defl;
-        const unsigned char *__restrict__ zr = defl ? d.defl_z + c0 : nullptr;
-        if (st.snorm_exit) {
-            const X_T wz = defl ? (X_T)(st.alpha * st.defl_cp) : X_T(0);
-            for (int base = threadIdx.x; base < np; base += U2 * blockDim.x) {
-                vec2_t<X_T> xv[U2];
-                vec2_t<T> pv[U2];
-#pragma unroll
-                for (int u = 0; u < U2; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        xv[u] = xload(q);
-                        pv[u] = ld2(ph + 2 * q);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U2; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        vec2_t<X_T> xn = mk2<X_T>(xv[u].x + alpha * (X_T)pv[u].x, xv[u].y + alpha * (X_T)pv[u].y);
-                        if (defl) {
-                            const uchar2 zz = *reinterpret_cast<const uchar2 *>(zr + 2 * q);
-                            if (zz.x) xn.x = xn.x + wz;
-                            if (zz.y) xn.y = xn.y + wz;
-                        }
-                        xstore(q, xn);
-                    }
-                }
-            }
-            if (!MIXED && (cnt & 1) && threadIdx.x == 0) x[cnt - 1] = x[cnt - 1] + alpha * (X_T)ph[cnt - 1];
-        } else {
-            const X_T omega = (X_T)st.omega;
-            const X_T wz = defl ? (X_T)(st.alpha * st.defl_cp + st.omega * st.defl_cs) : X_T(0);
-            const T omega_t = (T)st.omega;
-            const T *__restrict__ sh = vec<T>(d, sh_id) + c0;
-            const T *__restrict__ s = vec<T>(d, V_S) + c0;
-            const T *__restrict__ tv = vec<T>(d, V_T) + c0;
-            const T *__restrict__ rt = vec<T>(d, V_RT) + c0;
-            T *__restrict__ r = vec<T>(d, V_R) + c0;
-            for (int base = threadIdx.x; base < np; base += U2 * blockDim.x) {
-                vec2_t<X_T> xv[U2];
-                vec2_t<T> pv[U2], hv[U2], sv[U2], tw[U2], rtv[U2];
-#pragma unroll
-                for (int u = 0; u < U2; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        xv[u] = xload(q);
-                        pv[u] = ld2(ph + 2 * q);
-                        hv[u] = ld2(sh + 2 * q);
-                        sv[u] = ld2(s + 2 * q);
-                        tw[u] = ld2(tv + 2 * q);
-                        rtv[u] = ld2(rt + 2 * q);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < U2; ++u) {
-                    const int q = base + u * blockDim.x;
-                    if (q < np) {
-                        vec2_t<X_T> xn = mk2<X_T>(xv[u].x + alpha * (X_T)pv[u].x + omega * (X_T)hv[u].x,
-                                                  xv[u].y + alpha * (X_T)pv[u].y + omega * (X_T)hv[u].y);
-                        if (defl) {
-                            const uchar2 zz = *reinterpret_cast<const uchar2 *>(zr + 2 * q);
-                            if (zz.x) xn.x = xn.x + wz;
-                            if (zz.y) xn.y = xn.y + wz;
-                        }
-                        xstore(q, xn);
-                        const T r0 = sv[u].x - omega_t * tw[u].x, r1 = sv[u].y - omega_t * tw[u].y;
-                        st2(r + 2 * q, mk2<T>(r0, r1));
-                        v[0] += (double)r0 * (double)r0;
-                        v[1] += (double)rtv[u].x * (double)r0;
-                        v[0] += (double)r1 * (double)r1;
-                        v[1] += (double)rtv[u].y * (double)r1;
-                    }
-                }
-            }
-            if (!MIXED && (cnt & 1) && threadIdx.x == 0) {
-                const int c = cnt - 1;
-                x[c] = x[c] + alpha * (X_T)ph[c] + omega * (X_T)sh[c];
-                const T rv = s[c] - omega_t * tv[c];
-                r[c] = rv;
-                v[0] += (double)rv * (double)rv;
-                v[1] += (double)rt[c] * (double)rv;
-            }
-        }
+        xr_tile<T, MIXED, U2>(d, st, ph_id, sh_id, tl.idx, v);
         tile_partial<2>(b, d, tl.idx, v);
         run_add<2>(b, run, tl.sys, fin);
     }
@@ -1930,6 +1977,46 @@ __device__ __forceinline__ bool block_has_work(const BatchView &b, int gate)
     return __syncthreads_or(any) != 0;
 }
 
+// One tile of the FP64 reliable update, U cells per thread and pass.
+template <int U>
+__device__ __forceinline__ void outer_tile(const SysDev &d, const SysState &st, int idx, double (&v)[2])
+{
+    const int64_t c0 = (int64_t)idx * TILE_CELLS;
+    const int cnt = (int)min((int64_t)TILE_CELLS, d.n - c0);
+    const double *__restrict__ x = d.x64[0];
+    const bool fresh = (st.outer_steps == 0) || st.restart;
+    float *__restrict__ r32 = vec<float>(d, V_R);
+    float *__restrict__ rt32 = vec<float>(d, V_RT);
+    for (int base = threadIdx.x; base < cnt; base += U * blockDim.x) {
+        Row7<double> rw[U];
+        double bv[U];
+        float rtv[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = base + u * blockDim.x;
+            if (c < cnt) {
+                load_row7<double, double>(d, d.a64, x, c0 + c, rw[u]);
+                bv[u] = d.b64[c0 + c];
+                rtv[u] = fresh ? 0.f : rt32[padded(d, c0 + c)];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int c = base + u * blockDim.x;
+            if (c < cnt) {
+                const double rv = bv[u] - dot_row7<double>(rw[u], d.do_k);
+                const float rf = (float)rv;
+                const int64_t pc = padded(d, c0 + c);  // the FP32 vectors are padded
+                r32[pc] = rf;
+                const float rtf = fresh ? rf : rtv[u];
+                if (fresh) rt32[pc] = rf;
+                v[0] += rv * rv;
+                v[1] += (double)rtf * (double)rf;
+            }
+        }
+    }
+}
+
 __global__ void __launch_bounds__(256) k_outer_step(BatchView b)
 {
     constexpr int U = 2;
@@ -1942,41 +2029,8 @@ __global__ void __launch_bounds__(256) k_outer_step(BatchView b)
         const SysDev &d = b.sys[tl.sys];
         SysState &st = b.st[tl.sys];
         if (!gate_ok(st, G_OUTER)) continue;
-        const int64_t c0 = (int64_t)tl.idx * TILE_CELLS;
-        const int cnt = (int)min((int64_t)TILE_CELLS, d.n - c0);
-        const double *__restrict__ x = d.x64[0];
-        const bool fresh = (st.outer_steps == 0) || st.restart;
-        float *__restrict__ r32 = vec<float>(d, V_R);
-        float *__restrict__ rt32 = vec<float>(d, V_RT);
         double v[2] = {0.0, 0.0};
-        for (int base = threadIdx.x; base < cnt; base += U * blockDim.x) {
-            Row7<double> rw[U];
-            double bv[U];
-            float rtv[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int c = base + u * blockDim.x;
-                if (c < cnt) {
-                    load_row7<double, double>(d, d.a64, x, c0 + c, rw[u]);
-                    bv[u] = d.b64[c0 + c];
-                    rtv[u] = fresh ? 0.f : rt32[padded(d, c0 + c)];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                const int c = base + u * blockDim.x;
-                if (c < cnt) {
-                    const double rv = bv[u] - dot_row7<double>(rw[u], d.do_k);
-                    const float rf = (float)rv;
-                    const int64_t pc = padded(d, c0 + c);  // the FP32 vectors are padded
-                    r32[pc] = rf;
-                    const float rtf = fresh ? rf : rtv[u];
-                    if (fresh) rt32[pc] = rf;
-                    v[0] += rv * rv;
-                    v[1] += (double)rtf * (double)rf;
-                }
-            }
-        }
+        outer_tile<U>(d, st, tl.idx, v);
         tile_partial<2>(b, d, tl.idx, v);
         run_add<2>(b, run, tl.sys, fin);
     }
@@ -2134,7 +2188,7 @@ __device__ __forceinline__ bool next_line_job(const BatchView &b, const WaveArgs
                                               int lane, int vw, bool padded, int kind, LineJob &j, int pf = -1)
 {
     for (; item < total; item += step, pf = -1) {
-        const int sidx = (w.kind == 0) ? (pf >= 0 ? pf : __ldg(b.line_sys + item)) : 0;
+        const int sidx = (w.kind == 0 && b.nsys > 1) ? (pf >= 0 ? pf : __ldg(b.line_sys + item)) : 0;
         if (!gate_ok(b.st[sidx], w.gate)) continue;
         const SysDev &d = b.sys[sidx];
         if (d.line_kind != kind) continue;
@@ -2370,7 +2424,7 @@ __device__ __forceinline__ void line_recurrences(T *f, const T *fl, const T *fr,
 }
 
 template <typename T, int VW>
-__global__ void __launch_bounds__(128, sizeof(T) == 4 ? (VW == 4 ? 5 : 6) : 4) k_jline(BatchView b, WaveArgs w, int cmax)
+__device__ __forceinline__ void jline_body(const BatchView &b, const WaveArgs &w, int cmax, int block, int blocks)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int nwarps = blockDim.x >> 5;
@@ -2380,13 +2434,13 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? (VW == 4 ? 5 : 6) : 4) k
     T *s_l = s_f + rows_w, *s_r = s_l + rows_w, *s_q = s_r + rows_w;
 
     const int total = (w.kind == 0) ? b.line_prefix[b.nsys] : w.count;
-    const int step = gridDim.x * nwarps;
+    const int step = blocks * nwarps;
     LineJob j;
     int pf = -1;
-    for (int item = blockIdx.x * nwarps + warp; next_line_job(b, w, item, step, total, lane, VW, sizeof(T) == 4, LK_WARP, j, pf);
+    for (int item = block * nwarps + warp; next_line_job(b, w, item, step, total, lane, VW, sizeof(T) == 4, LK_WARP, j, pf);
          item = j.item + step) {
         // the next item's system, loaded while this one is processed
-        pf = (w.kind == 0 && j.item + step < total) ? __ldg(b.line_sys + j.item + step) : -1;
+        pf = (w.kind == 0 && b.nsys > 1 && j.item + step < total) ? __ldg(b.line_sys + j.item + step) : -1;
         const SysDev &d = b.sys[j.sidx];
         SysState &st = b.st[j.sidx];
         const LineCtx<T> x = line_ctx<T>(b, w, j);
@@ -2541,6 +2595,12 @@ __global__ void __launch_bounds__(128, sizeof(T) == 4 ? (VW == 4 ? 5 : 6) : 4) k
         }
         __syncwarp();
     }
+}
+
+template <typename T, int VW>
+__global__ void __launch_bounds__(128, sizeof(T) == 4 ? (VW == 4 ? 5 : 6) : 4) k_jline(BatchView b, WaveArgs w, int cmax)
+{
+    jline_body<T, VW>(b, w, cmax, blockIdx.x, gridDim.x);
 }
 
 // A line on which DGTSV interchanges rows or meets a zero pivot, solved by one
@@ -3020,6 +3080,275 @@ __global__ void __launch_bounds__(128, NP == 1 ? 3 : 2) k_jline_reg(const BatchV
             reg_line<T, NP>(b, w, c, sys, s_tail[warp], i, k, valid);
         }
         sys = next;
+    }
+}
+
+// ------------------------------------------------------------------ small batches: whole iterations in one launch
+// A 66^3-cell system's kernels have 2-3 us of work each; a launch, its ramp, its drain
+// and the chain of table, state and reduction accesses through L2 cost 4-8 us more:
+// the thirteen launches of a mixed iteration took 99 us there.  k_iterate runs whole
+// iterations in one cooperative launch: every block owns a cell tile (or none: SMs left
+// over) and a share of the lines of one system, whose fields and scalars it keeps in
+// shared memory, and a system's blocks meet at a barrier of their own between steps.  Every block of a
+// system adds the same partial sums in the same order and takes the same scalar
+// steps, so none waits for another's scalars, and the results are the bits of the
+// launches.  A system's blocks leave when it is done or after the asked number of
+// iterations; waits are bounded, and a block that gives up sets *IterArgs::abort and
+// error flag 4 of its system.
+__device__ __forceinline__ unsigned ld_relaxed(const unsigned *p)
+{
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
+{
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void red_release_add(unsigned *p, unsigned v)
+{
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory");
+}
+
+// The n blocks of a system (all resident: the launch is cooperative) arrive before
+// one leaves; what they wrote before is visible after.  `target` counts the arrivals
+// so far.  False when the wait ran out of time (about two seconds).
+__device__ __forceinline__ bool group_barrier(GroupBar *g, unsigned n, unsigned &target, unsigned *abort)
+{
+    __shared__ int ok;
+    __syncthreads();
+    target += n;
+    if (threadIdx.x == 0) {
+        red_release_add(&g->count, 1u);
+        bool in_time = true;
+        if (ld_acquire(&g->count) < target) {  // an acquire drops the SM's L1 lines: the waiting itself reads relaxed
+            const long long t0 = clock64();
+            for (int q = 1; in_time && ld_relaxed(&g->count) < target; ++q)
+                if ((q & 63) == 0) in_time = clock64() - t0 < (1LL << 32) && ld_relaxed(abort) == 0u;
+            ld_acquire(&g->count);
+        }
+        if (!in_time) atomicExch(abort, 1u);
+        ok = in_time;
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+// One cell step of k_iterate on the block's tile, its sums to the tile's slot.  Few
+// cells per thread and pass: with more the kernel spills (two cell pairs in the
+// matvecs: 684 bytes a thread), and as functions of their own the steps took 16,200
+// cycles a tile, most of it saving registers, against 8,100.
+enum : int { IT_OUTER, IT_P, IT_ALPHA, IT_S, IT_OMEGA, IT_XR };
+template <int NV>
+__device__ __forceinline__ void store_sums(double (&v)[NV], double *slot)
+{
+    block_sum<NV>(v);
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int q = 0; q < NV; ++q) slot[q] = v[q];
+}
+template <typename T, bool MIXED, int STEP>
+__device__ __forceinline__ bool iterate_cells(const SysDev &d, const SysState &st, int idx, double *slot)
+{
+    constexpr int MVP = 1, ST = sizeof(T) == 4 ? 4 : 2, XR = 1;
+    constexpr int NV = STEP == IT_P || STEP == IT_ALPHA || (STEP == IT_S && !MIXED) ? 1 : 2;
+    double v[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q] = 0.0;
+    if constexpr (STEP == IT_OUTER) outer_tile<1>(d, st, idx, v);
+    if constexpr (STEP == IT_P)
+        if (!p_tile<T, MIXED, ST>(d, st, idx, v)) return false;
+    if constexpr (STEP == IT_ALPHA || STEP == IT_OMEGA) {
+        if constexpr (sizeof(T) == 8) {
+            if (!pair_rows<T>(d)) {
+                if constexpr (STEP == IT_ALPHA) alpha_tile<T, MIXED, false, 1, 1>(d, st, V_PH, idx, v);
+                if constexpr (STEP == IT_OMEGA) omega_tile<T, MIXED, false, 1, 1>(d, st, V_SH, idx, v);
+                store_sums<NV>(v, slot);
+                return true;
+            }
+        }
+        if constexpr (STEP == IT_ALPHA) alpha_tile<T, MIXED, true, 1, MVP>(d, st, V_PH, idx, v);
+        if constexpr (STEP == IT_OMEGA) omega_tile<T, MIXED, true, 1, MVP>(d, st, V_SH, idx, v);
+    }
+    if constexpr (STEP == IT_S) s_tile<T, MIXED, ST>(d, st, idx, v);
+    if constexpr (STEP == IT_XR) xr_tile<T, MIXED, XR>(d, st, V_PH, V_SH, idx, v);
+    store_sums<NV>(v, slot);
+    return true;
+}
+// One half-sweep over the block's share of the system's lines.
+constexpr int IT_WARPS = 8;
+template <typename T>
+__device__ __forceinline__ void iterate_lines(const BatchView &b, const BatchView &own, const SysDev &d, const LineSys &c,
+                                           const WaveArgs &w, int sys, int idx, int blocks, int cmax, unsigned char *tails)
+{
+    if (d.line_kind == LK_REG) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lpw = 5 - c.lg;
+        const int items = (d.half_lines * d.kmax2 + (1 << lpw) - 1) >> lpw;
+        for (int item = idx * IT_WARPS + warp; item < items; item += blocks * IT_WARPS) {
+            int i, k;
+            const bool valid = wave_line(d, w, (item << lpw) + (lane >> c.lg), i, k);
+            if (!valid) i = k = 1;  // reads line (1, 1) and stores nothing
+            reg_line<T, 1>(b, w, c, sys, tails + warp * (LR_N + 4) * LINE_TAIL, i, k, valid);
+        }
+    } else {
+        jline_body<T, sizeof(T) == 4 ? 2 : 1>(own, w, cmax, idx, blocks);
+    }
+}
+
+template <typename T, bool MIXED>
+__global__ void __launch_bounds__(32 * IT_WARPS, 1) k_iterate(const BatchView b, const IterArgs a)
+{
+    __shared__ SysDev d;
+    __shared__ SysState st;
+    __shared__ LineSys line;
+    __shared__ WaveArgs w;
+    __shared__ BatchView view, own;  // the batch, and the system alone
+    __shared__ int prefix[2];
+    __shared__ __align__(16) unsigned char tails[IT_WARPS * (LR_N + 4) * LINE_TAIL];
+    const IterBlock mine = a.blocks[blockIdx.x];
+    const int sys = mine.sys, idx = mine.idx;
+    for (int q = threadIdx.x; q < (int)(sizeof(SysDev) / 8); q += blockDim.x)
+        reinterpret_cast<uint64_t *>(&d)[q] = reinterpret_cast<const uint64_t *>(b.sys + sys)[q];
+    for (int q = threadIdx.x; q < (int)(sizeof(SysState) / 8); q += blockDim.x)
+        reinterpret_cast<uint64_t *>(&st)[q] = reinterpret_cast<const uint64_t *>(b.st + sys)[q];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int q = LR_L; q < LR_M0; ++q) line.arr[q] = reinterpret_cast<const char *>(d.fac[q - LR_L]);
+        const int diag[4] = {2, 4, 0, 6};  // A(-1), A(1), A(-3), A(3)
+        for (int q = 0; q < 4; ++q)
+            line.arr[LR_M0 + q] = reinterpret_cast<const char *>(diag_base<T>(d) + (int64_t)diag[q] * cells<T>(d));
+        line.c1 = pitch<T>(d) * (int)sizeof(T);
+        line.c2 = (int64_t)line.c1 * d.imax2;
+        line.g0 = 0;
+        line.lg = 31 - __clz(d.lane_group);
+        line.np = d.line_np;
+        line.rows = pitch<T>(d);
+        line.extra = 32 / (int)sizeof(T) * d.lane_group * d.line_np < d.jmax2;
+        line.imax2 = d.imax2;
+        line.kmax2 = d.kmax2;
+        line.do_k = d.do_k;
+        line.cyc = d.cyc;
+        line.flags = d.line_flag;
+        const int lpw = 32 / d.lane_group;
+        prefix[0] = 0;
+        prefix[1] = (d.half_lines * d.kmax2 + lpw - 1) / lpw;
+        view = own = b;
+        own.sys = &d;
+        own.st = b.st + sys;
+        own.nsys = 1;
+        own.line_prefix = prefix;
+    }
+    __syncthreads();
+    GroupBar *bar = a.bar + sys;
+    const unsigned n = (unsigned)mine.count;
+    const bool tiled = idx < d.ntiles;
+    unsigned target = 0;
+    int parity = 0;  // of the partial sums' two sets: a block may be one step ahead of another's reads
+    bool fine = ld_relaxed(a.abort) == 0u;
+    auto sync = [&]() {
+        if (fine) fine = group_barrier(bar, n, target, a.abort);
+    };
+    auto sums = [&]() -> double * { return b.partials + 2 * ((int64_t)parity * b.ntiles + d.tile_base); };
+    // the system's totals from its tiles' slots, as run_close adds them, and the scalar step
+    auto reduce = [&](auto nv, auto &&fin) {
+        constexpr int NV = decltype(nv)::value;
+        sync();
+        if (!fine) return;
+        double acc[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) acc[q] = 0.0;
+        const double *from = sums();
+        for (int t = threadIdx.x; t < d.ntiles; t += blockDim.x)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) acc[q] += __ldcg(from + 2 * t + q);
+        block_sum<NV>(acc);
+        if (threadIdx.x == 0) fin(st, acc);
+        parity ^= 1;
+        __syncthreads();
+    };
+    using One = std::integral_constant<int, 1>;
+    using Two = std::integral_constant<int, 2>;
+    using Snorm = std::integral_constant<int, MIXED ? 2 : 1>;
+    // LEQ_MSOLVE with R letters (Engine::plan_msolve's waves)
+    auto msolve = [&](int src, int dst) {
+        for (int s = 0; s < a.ns && fine; ++s) {
+            if (threadIdx.x == 0) {
+                w = WaveArgs{};
+                w.par = (s & 1) ^ 1;
+                w.rhs = src;
+                w.dst = dst;
+                w.nbr = s == 0 ? src : dst;
+                w.old = s <= 1 ? src : dst;
+                w.write_old = s <= 1;
+                w.gate = G_ANY;
+                line.arr[LR_F] = reinterpret_cast<const char *>(vec<T>(d, src));
+                line.nbr = reinterpret_cast<const char *>(vec<T>(d, w.nbr));
+                line.old = reinterpret_cast<const char *>(vec<T>(d, w.old));
+                line.dst = reinterpret_cast<char *>(vec<T>(d, dst));
+            }
+            __syncthreads();
+            iterate_lines<T>(view, own, d, line, w, sys, idx, (int)n, a.line_cmax, tails);
+            sync();
+        }
+    };
+    for (int it = 0; it < a.iterations && fine && st.status == ST_RUNNING; ++it) {
+        if constexpr (MIXED) {
+            if (st.phase == PH_OUTER) {
+                if (tiled) iterate_cells<T, MIXED, IT_OUTER>(d, st, idx, sums() + 2 * idx);
+                reduce(Two{}, [](SysState &q, const double(&t)[2]) { fin_outer(q, t[0], t[1]); });
+            }
+            if (!fine || st.status != ST_RUNNING || st.phase != PH_INNER) continue;
+        }
+        bool summed = MIXED && st.defl;
+        if (tiled) summed = iterate_cells<T, MIXED, IT_P>(d, st, idx, sums() + 2 * idx);
+        if (summed)
+            reduce(One{}, [](SysState &q, const double(&t)[1]) { fin_p(q, t); });
+        else
+            sync();
+        msolve(V_P, V_PH);
+        if (!fine) break;
+        if (tiled) iterate_cells<T, MIXED, IT_ALPHA>(d, st, idx, sums() + 2 * idx);
+        reduce(One{}, [](SysState &q, const double(&t)[1]) { fin_alpha(q, t); });
+        if (!fine) break;
+        if (tiled) iterate_cells<T, MIXED, IT_S>(d, st, idx, sums() + 2 * idx);
+        reduce(Snorm{}, [](SysState &q, const double(&t)[MIXED ? 2 : 1]) { fin_s<MIXED>(q, t); });
+        if (!fine) break;
+        if (!st.snorm_exit) {
+            msolve(V_S, V_SH);
+            if (!fine) break;
+            if (tiled) iterate_cells<T, MIXED, IT_OMEGA>(d, st, idx, sums() + 2 * idx);
+            reduce(Two{}, [](SysState &q, const double(&t)[2]) { fin_omega(q, t); });
+            if (!fine) break;
+        }
+        if (tiled) iterate_cells<T, MIXED, IT_XR>(d, st, idx, sums() + 2 * idx);
+        reduce(Two{}, [](SysState &q, const double(&t)[2]) {
+            if (MIXED)
+                fin_xr_inner(q, t[0], t[1]);
+            else
+                fin_xr_ref(q, t[0], t[1]);
+        });
+    }
+    __syncthreads();
+    SysState &out = b.st[sys];
+    if (!fine) {
+        if (threadIdx.x == 0) atomicOr(&out.err, 4);
+    } else if (idx == 0) {  // the state back, with the counts the line kernels keep in it
+        if (threadIdx.x == 0) {
+            st.err |= out.err;
+            st.line_skips = __ldcg(&out.line_skips);
+            st.line_fallbacks = __ldcg(&out.line_fallbacks);
+            st.arrivals = 0;
+        }
+        __syncthreads();
+        for (int q = threadIdx.x; q < (int)(sizeof(SysState) / 8); q += blockDim.x)
+            reinterpret_cast<uint64_t *>(&out)[q] = reinterpret_cast<const uint64_t *>(&st)[q];
+    }
+    // the system's last block to leave readies its barrier for the next launch
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicInc(&bar->left, n - 1) == n - 1) bar->count = 0u;
     }
 }
 
@@ -3745,6 +4074,33 @@ cudaError_t launch_jline(const BatchView &b, const LaunchCfg &c, const WaveArgs 
     }
     CHECK_LAUNCH();
 }
+// Dynamic shared memory of k_iterate: k_jline's rows of its warps.
+template <typename T>
+static int iterate_smem(const IterArgs &a)
+{
+    return a.line_warp ? IT_WARPS * kernel_smem_line_bytes(a.line_cmax, (int)sizeof(T)) : 0;
+}
+
+template <typename T, bool MIXED>
+bool iterate_fits(const IterArgs &a)
+{
+    constexpr int MOST = 180 * 1024;  // beside the static 16 KB
+    static const bool ready = cudaFuncSetAttribute(k_iterate<T, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   MOST) == cudaSuccess;
+    cudaGetLastError();
+    return ready && iterate_smem<T>(a) <= MOST;
+}
+
+template <typename T, bool MIXED>
+cudaError_t launch_iterate(const BatchView &b, const LaunchCfg &c, const IterArgs &a)
+{
+    BatchView bv = b;
+    IterArgs av = a;
+    void *args[] = {&bv, &av};
+    return cudaLaunchCooperativeKernel((const void *)k_iterate<T, MIXED>, dim3(a.nblocks), dim3(32 * IT_WARPS), args,
+                                       (size_t)iterate_smem<T>(a), c.stream);
+}
+
 template <typename T>
 cudaError_t launch_diag(const BatchView &b, const LaunchCfg &c, int src, int dst, int gate)
 {
@@ -3868,6 +4224,8 @@ cudaError_t launch_seq_lines(const BatchView &b, const SeqLineArgs &a, cudaStrea
     template cudaError_t launch_p_update<T, M>(const BatchView &, const LaunchCfg &);       \
     template cudaError_t launch_matvec_alpha<T, M>(const BatchView &, const LaunchCfg &, int); \
     template cudaError_t launch_s_update<T, M>(const BatchView &, const LaunchCfg &);       \
+    template bool iterate_fits<T, M>(const IterArgs &);                                     \
+    template cudaError_t launch_iterate<T, M>(const BatchView &, const LaunchCfg &, const IterArgs &); \
     template cudaError_t launch_matvec_omega<T, M>(const BatchView &, const LaunchCfg &, int); \
     template cudaError_t launch_xr_update<T, M>(const BatchView &, const LaunchCfg &, int, int);
 INST_T(double)

@@ -15,7 +15,7 @@ struct BatchView {
     const int *line_sys;     // [items] the system of each of them
     const int *reg_prefix;   // the same of k_jline_reg
     const int *reg_sys;
-    double *partials;        // [ntiles_total * 2]
+    double *partials;        // [ntiles_total * 2], and a second set of them (k_iterate)
 };
 
 struct LaunchCfg {
@@ -89,6 +89,12 @@ template <typename T>
 cudaError_t launch_copy(const BatchView &b, const LaunchCfg &c, int src, int dst, int gate);
 template <typename T, bool MIXED>
 cudaError_t launch_matvec_alpha(const BatchView &b, const LaunchCfg &c, int src);   // V = A*Phat, alpha
+// Whole iterations of a small batch in one cooperative launch (at most one block per
+// SM); whether the device can run it.
+template <typename T, bool MIXED>
+bool iterate_fits(const IterArgs &a);
+template <typename T, bool MIXED>
+cudaError_t launch_iterate(const BatchView &b, const LaunchCfg &c, const IterArgs &a);
 template <typename T, bool MIXED>
 cudaError_t launch_s_update(const BatchView &b, const LaunchCfg &c);               // S = R - alpha V, Snorm
 template <typename T, bool MIXED>

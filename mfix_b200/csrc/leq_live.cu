@@ -256,7 +256,7 @@ int Engine::live_commit()
     CK(upload_staged(&d_tiles_, &tiles_cap_, h_tiles_.data(), h_tiles_.size()));
     CK(upload_staged(&d_allprefix_, &allprefix_cap_, h_allprefix_.data(), h_allprefix_.size()));
     CK(stage_close());
-    const size_t need_part = 2 * (size_t)std::max(tile_base, 1);
+    const size_t need_part = 4 * (size_t)std::max(tile_base, 1);  // two sets of partial sums
     if (need_part > part_cap_) {
         cudaFree(d_partials_);  // waits for the kernels that still use it
         d_partials_ = nullptr;
@@ -300,7 +300,8 @@ int Engine::live_commit()
     // the iteration body for this membership
     if (live_exec_) retired_execs_.push_back({live_exec_, snap_count_});  // its launches may still run
     live_exec_ = nullptr;
-    if (live_used_ > 0 && live_opt_.use_graph) {
+    live_small_ = live_used_ > 0 && small_batch(live_opt_, &live_iter_);
+    if (live_used_ > 0 && live_opt_.use_graph && !live_small_) {
         cudaGraph_t g = nullptr;
         CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
         const long long before = launches_;
@@ -338,7 +339,8 @@ int Engine::live_step(int iterations)
     CK(cudaEventRecord(ev_c0_[b], stream_));
     if (live_dirty_ && (rc = live_commit())) return rc;
     if (live_used_ == 0 || iterations <= 0) return 0;
-    for (int q = 0; q < iterations; ++q) {
+    if (live_small_) CK(run_iterations(live_opt_, live_iter_, iterations));
+    for (int q = 0; q < iterations && !live_small_; ++q) {
         if (live_exec_) {
             CK(cudaGraphLaunch(live_exec_, stream_));
             launches_ += live_per_body_;
@@ -401,6 +403,7 @@ int Engine::live_take(long long q, std::vector<LiveDone> &done)
     for (int s = 0; s < cap; ++s) {
         if (!slot_used_[s] || slot_reported_[s] || slot_fresh_[s] || q < slot_join_snap_[s]) continue;
         const SysState &st = ps[s];
+        bar_dirty_ = bar_dirty_ || (st.err & 4);
         // a system still running after ITMAX + 2 bodies is reported incomplete, as
         // the one-shot solve reports it
         if (st.status != ST_RUNNING || snap_bodies_[b] - slot_join_body_[s] >= (long long)st.itmax + 2) {
