@@ -603,8 +603,9 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
         }
         return (size_t)kernel_smem_line_bytes(rows_for(L, 32), elem) <= 48 * 1024 ? (np > 0 ? 32 | LINE_STAGED : 32) : 0;
     };
-    bool any_reg = false, any_long = false;
+    bool any_reg = false, any_long = false, one_pass = true;
     for (int L : todo) {
+        one_pass = one_pass && reg_passes(L, elem, 32) == 1;
         any_reg = any_reg || reg_passes(L, elem, 32) > 0;
         any_long = any_long || L > 32;
     }
@@ -628,11 +629,19 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
     float best_ms = 1e30f;
     // the register kernel's one shape first (the fewest lanes that hold a line in its
     // fewest passes: more lanes idle), then k_jline at every width, which has to be 5%
-    // faster where the register kernel serves the batch (60.6 us against 66.1 for four
+    // faster where the register kernel serves the batch (62-63 us against 66 for four
     // FP32 half-sweeps of 145x173x100 cells, 336 against 290 of 258^3): k_iterate, which
     // has few warps, prefers the shape with the most lines a warp.  One lane per line
     // for short lines only (at 66 cells it takes nine times the best width's time).
-    for (int cand = any_reg ? -1 : any_long ? 1 : 0; cand < 6; ++cand) {
+    // A batch small enough for k_iterate launches sweeps of 3-4 us, which all time alike
+    // (26 to 35 us for four at 66^3 to 80^3 cells, the choice a matter of chance): there the
+    // register kernel is taken without a timing where it serves every line in one pass
+    // (60 iterations at 74^3: FP32 12.9 ms with k_jline's shape, 9.6 with this one, FP64
+    // 6.5 and 5.4), and elsewhere a wider shape has to be 5% faster (FP64 at 65^3: 5.1 ms
+    // with 16 lanes, 6.1 with 32).
+    const bool small = view_.ntiles <= sms_;
+    const int cand_end = small && one_pass ? 0 : 6;
+    for (int cand = any_reg ? -1 : any_long ? 1 : 0; cand < cand_end; ++cand) {
         if (any_reg && cand == 0) continue;
         const int g = cand < 0 ? 2 : 1 << cand;
         const bool staged = cand > 0 && any_reg;
@@ -654,7 +663,7 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
         CK(cudaEventRecord(e1, stream_));
         CK(cudaEventSynchronize(e1));
         cudaEventElapsedTime(&tot, e0, e1);
-        if (tot < (staged && !best_staged ? 0.95f : 1.f) * best_ms) {
+        if (tot < (small || (staged && !best_staged) ? 0.95f : 1.f) * best_ms) {
             best_ms = tot;
             best_g = g;
             best_staged = staged;
