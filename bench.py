@@ -647,7 +647,7 @@ def run_ours(args) -> None:
     avg_launch_s = (jl_ms / 1e3) / max(jl_work, 1)
     achieved = alg_bytes_launch / avg_launch_s / 1e9
     traffic = ncu_traffic(f"jline_f32_{w}.md")
-    roof = {"kernel": "k_jline<float> (LINE preconditioner half-sweep)", "bound": "hbm", "achieved": achieved,
+    roof = {"kernel": "k_jline_reg<float, NP> (LINE preconditioner half-sweep)", "bound": "hbm", "achieved": achieved,
             "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_kind": f"{peak_kind} (MEASURED_PEAKS hbm_gbs)",
             "alg_bytes_per_launch": alg_bytes_launch, "avg_launch_ms": avg_launch_s * 1e3, "launches": jl_n,
             "work_launches": jl_work, "traffic": traffic}
@@ -812,7 +812,7 @@ def run_cg_bench(args) -> None:
         "config": {"workload": w, "grid": list(WORKLOADS[w]["dims"]), "cells": n, "method": 5, "pc": "LINE",
                    "sweep": "RSRS", "tol": sys0.tol, "itmax": sys0.itmax,
                    "l2_policy": "inputs larger than L2 (A_M 7*8*cells bytes), no flush needed"},
-        "roofline": {"kernel": "k_jline<double> (LINE preconditioner half-sweep)", "bound": "hbm",
+        "roofline": {"kernel": "k_jline_reg<double, NP> (LINE preconditioner half-sweep)", "bound": "hbm",
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "alg_bytes_per_launch": alg_launch, "avg_launch_ms": avg_s * 1e3,
                      "launches": jl_n, "work_launches": jl_work, "traffic": ncu_traffic(f"jline_f64_{w}.md")},

@@ -2341,7 +2341,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // VW rows per access: a lane reads VW consecutive rows of each operand with one
 // load (16 bytes for VW = 4 in FP32 and VW = 2 in FP64), which needs lines that
 // start on VW-row boundaries (the mixed form's padded FP32 arrays, pitch a
-// multiple of four; an even JMAX2 for two rows).
+// multiple of eight; an even JMAX2 for two rows).
 template <typename T, int VW>
 struct alignas(VW * sizeof(T)) RowsV {
     T v[VW];
