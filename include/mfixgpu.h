@@ -181,6 +181,8 @@ const char *mfixgpu_last_error(void);
  *   "use_graph"      1 (default) replay the iteration body as a CUDA graph, or run the iterations of a
  *                    small batch (at most one cell tile per SM) in one cooperative launch; 0: launch
  *                    every kernel by itself (the same bits)
+ *   "wait_polls"     reads a block of that launch makes at a barrier before it gives up and its system
+ *                    returns IER -15 (default 2^22, a second or two; 0..1e9)
  *   "time_kernels"   1: time every J-line sweep launch with CUDA events (no graph replay)
  *   "autotune"       1 (default): lanes per J-line picked by measurement for the new line lengths of a
  *                    solve or batch (one lanes-per-line value timed on all their lines at once)

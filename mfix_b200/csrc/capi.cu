@@ -43,6 +43,7 @@ struct Options {
     int staged_matvec = 2;
     int do_transpose = 0;
     int check_every = 4;
+    unsigned wait_polls = 1u << 22;
     int use_graph = 1;
     int time_kernels = 0;
     int autotune = 1;
@@ -283,6 +284,7 @@ SolveOptions make_opts(const Options &o, int pc, const char sweep4[4])
     so.icheck_bicgs = o.icheck_bicgs;
     so.staged_matvec = o.staged_matvec;
     so.check_every = o.check_every;
+    so.wait_polls = o.wait_polls;
     so.use_graph = o.use_graph != 0;
     so.time_kernels = o.time_kernels != 0;
     so.autotune = o.autotune != 0;
@@ -698,6 +700,9 @@ int mfixgpu_set_option(const char *name, double value)
     } else if (k == "check_every") {
         if (value < 1) return MFIXGPU_ERR_ARGS;
         g.opt.check_every = (int)value;
+    } else if (k == "wait_polls") {
+        if (!(value >= 0 && value <= 1e9)) return MFIXGPU_ERR_ARGS;
+        g.opt.wait_polls = (unsigned)value;
     } else if (k == "use_graph") {
         g.opt.use_graph = value != 0;
     } else if (k == "time_kernels") {
@@ -734,6 +739,7 @@ double mfixgpu_get_option(const char *name)
     if (k == "icheck_bicgs") return g.opt.icheck_bicgs;
     if (k == "do_transpose") return g.opt.do_transpose;
     if (k == "check_every") return g.opt.check_every;
+    if (k == "wait_polls") return g.opt.wait_polls;
     if (k == "use_graph") return g.opt.use_graph;
     if (k == "time_kernels") return g.opt.time_kernels;
     if (k == "autotune") return g.opt.autotune;

@@ -191,8 +191,9 @@ struct WaveArgs {
 };
 
 // Arrivals of k_iterate's barrier of one system, kept on the device between launches.
+constexpr unsigned BAR_GAVE_UP = 0x80000000u;
 struct GroupBar {
-    unsigned count;  // blocks that have arrived, all barriers of the running launch
+    unsigned count;  // blocks that have arrived, all barriers of the running launch; BAR_GAVE_UP: a wait ran out
     unsigned pad0[31];
     unsigned left;   // blocks that have left the launch
     unsigned pad1[31];
@@ -212,7 +213,7 @@ struct IterArgs {
     int ns;          // half-sweeps per LEQ_MSOLVE
     int line_warp, line_cmax;  // as in LaunchCfg
     GroupBar *bar;   // [nsys]
-    unsigned *abort; // a wait ran out of time
+    unsigned polls;  // reads of the count a block makes at a barrier before it gives up
 };
 
 enum Gate : int {

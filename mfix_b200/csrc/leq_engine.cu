@@ -181,7 +181,7 @@ SolveResult result_of(const SysState &st, bool mixed)
         r.exit_kind = EX_ERROR;
     }
     if (st.err & 4) {
-        r.ier = -15;  // a staged copy did not complete within its time limit
+        r.ier = -15;  // a staged copy or a barrier of k_iterate did not complete within its limit
         r.exit_kind = EX_ERROR;
     }
     if (st.err & 2) {
@@ -1343,17 +1343,17 @@ bool Engine::small_batch(const SolveOptions &opt, IterArgs *a)
     a->line_warp = cfg_.line_warp;
     a->line_cmax = cfg_.line_cmax;
     if (!(opt.precision == PREC_MIXED ? iterate_fits<float, true>(*a) : iterate_fits<double, false>(*a))) return false;
-    if ((size_t)nsys_ + 1 > bar_cap_) {
+    if ((size_t)nsys_ > bar_cap_) {
         cudaFree(d_bar_);
         d_bar_ = nullptr;
         bar_cap_ = 0;
         bar_dirty_ = true;
-        if (cudaMalloc((void **)&d_bar_, sizeof(GroupBar) * ((size_t)nsys_ + 1)) != cudaSuccess) {
+        if (cudaMalloc((void **)&d_bar_, sizeof(GroupBar) * (size_t)nsys_) != cudaSuccess) {
             cudaGetLastError();
             d_bar_ = nullptr;
             return false;
         }
-        bar_cap_ = (size_t)nsys_ + 1;
+        bar_cap_ = (size_t)nsys_;
     }
     // a block per tile; the SMs left over go to the systems whose lines need more
     // rounds of a block's eight warps than one, in proportion to what they miss
@@ -1380,8 +1380,8 @@ bool Engine::small_batch(const SolveOptions &opt, IterArgs *a)
         return false;
     }
     a->blocks = d_iter_blocks_;
-    a->bar = d_bar_ + 1;
-    a->abort = &d_bar_->count;
+    a->bar = d_bar_;
+    a->polls = opt.wait_polls;
     return true;
 }
 
@@ -1495,11 +1495,7 @@ int Engine::run_batch(const std::vector<SystemSpec> &specs, const SolveOptions &
         CK(cudaEventRecord(ev_a_, stream_));
         CK(cudaEventSynchronize(ev_a_));
         finished = true;
-        for (int s = 0; s < nsys_; ++s) {
-            const SysState &st = h_st_pinned_[s];
-            finished = finished && (st.status != ST_RUNNING || (st.err & 4));
-            bar_dirty_ = bar_dirty_ || (st.err & 4);
-        }
+        for (int s = 0; s < nsys_; ++s) finished = finished && h_st_pinned_[s].status != ST_RUNNING;
     }
     while (!small && loops < max_loops && !finished) {
         for (int q = 0; q < K && loops < max_loops; ++q, ++loops)

@@ -73,6 +73,7 @@ struct SolveOptions {
     bool transposed = false;     // DO_TRANSPOSE (model/solve_lin_eq.f:139-150): LEQ_BICGSt's preconditioner
                                  // letters, and A is scaled in a copy (only B comes back scaled)
     int check_every = 4;         // iterations between host checks of the state
+    unsigned wait_polls = 1u << 22;  // reads of a barrier's count in k_iterate before a block gives up
     bool use_graph = true;       // capture the iteration body in a CUDA graph
     bool time_kernels = false;   // record events around every J-line launch (no graph replay)
     bool skip_scale = false;     // the system is unit-scaled already (FP64 re-solve after a mixed attempt)
@@ -313,9 +314,9 @@ private:
     std::vector<ListRef> list_refs_;
 
     // small batches: whole iterations in one cooperative launch (k_iterate)
-    GroupBar *d_bar_ = nullptr;  // one per system, then the abort word
+    GroupBar *d_bar_ = nullptr;  // one per system
     size_t bar_cap_ = 0;
-    bool bar_dirty_ = true;      // they have to be cleared before the next launch
+    bool bar_dirty_ = true;      // new: to be cleared before the first launch (each launch leaves them clear)
     std::vector<IterBlock> h_iter_blocks_;
     IterBlock *d_iter_blocks_ = nullptr;
     size_t iter_blocks_cap_ = 0;

@@ -3093,8 +3093,8 @@ __global__ void __launch_bounds__(128, NP == 1 ? 3 : 2) k_jline_reg(const BatchV
 // system adds the same partial sums in the same order and takes the same scalar
 // steps, so none waits for another's scalars, and the results are the bits of the
 // launches.  A system's blocks leave when it is done or after the asked number of
-// iterations; waits are bounded, and a block that gives up sets *IterArgs::abort and
-// error flag 4 of its system.
+// iterations.  Waits are bounded: a wait that runs out ends its own system with error
+// flag 4, in all its blocks (group_barrier), and no other.
 __device__ __forceinline__ unsigned ld_relaxed(const unsigned *p)
 {
     unsigned v;
@@ -3114,23 +3114,28 @@ __device__ __forceinline__ void red_release_add(unsigned *p, unsigned v)
 
 // The n blocks of a system (all resident: the launch is cooperative) arrive before
 // one leaves; what they wrote before is visible after.  `target` counts the arrivals
-// so far.  False when the wait ran out of time (about two seconds).
-__device__ __forceinline__ bool group_barrier(GroupBar *g, unsigned n, unsigned &target, unsigned *abort)
+// so far.  After `polls` reads of the count (an L2 round trip each; they stop while
+// another process has the GPU, which a clock would not) a block gives up, by a compare
+// and swap that fails when another has arrived since: so no barrier that gave up
+// completes later, and every block of the system sees the flag at this barrier or its
+// next.  False, in all threads, when the wait ran out here or in another block.
+__device__ __forceinline__ bool group_barrier(GroupBar *g, unsigned n, unsigned &target, unsigned polls)
 {
     __shared__ int ok;
     __syncthreads();
     target += n;
     if (threadIdx.x == 0) {
         red_release_add(&g->count, 1u);
-        bool in_time = true;
-        if (ld_acquire(&g->count) < target) {  // an acquire drops the SM's L1 lines: the waiting itself reads relaxed
-            const long long t0 = clock64();
-            for (int q = 1; in_time && ld_relaxed(&g->count) < target; ++q)
-                if ((q & 63) == 0) in_time = clock64() - t0 < (1LL << 32) && ld_relaxed(abort) == 0u;
+        unsigned seen = ld_acquire(&g->count);
+        if (seen < target) {  // an acquire drops the SM's L1 lines: the waiting itself reads relaxed
+            for (unsigned q = 0; (seen = ld_relaxed(&g->count)) < target; ++q)
+                if (q >= polls && atomicCAS(&g->count, seen, seen | BAR_GAVE_UP) == seen) {
+                    seen |= BAR_GAVE_UP;
+                    break;
+                }
             ld_acquire(&g->count);
         }
-        if (!in_time) atomicExch(abort, 1u);
-        ok = in_time;
+        ok = (seen & BAR_GAVE_UP) == 0u;
     }
     __syncthreads();
     return ok != 0;
@@ -3246,9 +3251,9 @@ __global__ void __launch_bounds__(32 * IT_WARPS, 1) k_iterate(const BatchView b,
     const bool tiled = idx < d.ntiles;
     unsigned target = 0;
     int parity = 0;  // of the partial sums' two sets: a block may be one step ahead of another's reads
-    bool fine = ld_relaxed(a.abort) == 0u;
+    bool fine = true;
     auto sync = [&]() {
-        if (fine) fine = group_barrier(bar, n, target, a.abort);
+        if (fine) fine = group_barrier(bar, n, target, a.polls);
     };
     auto sums = [&]() -> double * { return b.partials + 2 * ((int64_t)parity * b.ntiles + d.tile_base); };
     // the system's totals from its tiles' slots, as run_close adds them, and the scalar step
@@ -3332,11 +3337,14 @@ __global__ void __launch_bounds__(32 * IT_WARPS, 1) k_iterate(const BatchView b,
     }
     __syncthreads();
     SysState &out = b.st[sys];
-    if (!fine) {
-        if (threadIdx.x == 0) atomicOr(&out.err, 4);
-    } else if (idx == 0) {  // the state back, with the counts the line kernels keep in it
+    if (idx == 0) {  // the state back, with the counts the line kernels keep in it
         if (threadIdx.x == 0) {
-            st.err |= out.err;
+            st.err |= __ldcg(&out.err);
+            if (!fine) {  // vectors half updated: the system is over
+                st.err |= 4;
+                st.exit_kind = EX_ERROR;
+                st.status = ST_DONE;
+            }
             st.line_skips = __ldcg(&out.line_skips);
             st.line_fallbacks = __ldcg(&out.line_fallbacks);
             st.arrivals = 0;

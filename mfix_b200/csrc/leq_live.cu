@@ -403,7 +403,6 @@ int Engine::live_take(long long q, std::vector<LiveDone> &done)
     for (int s = 0; s < cap; ++s) {
         if (!slot_used_[s] || slot_reported_[s] || slot_fresh_[s] || q < slot_join_snap_[s]) continue;
         const SysState &st = ps[s];
-        bar_dirty_ = bar_dirty_ || (st.err & 4);
         // a system still running after ITMAX + 2 bodies is reported incomplete, as
         // the one-shot solve reports it
         if (st.status != ST_RUNNING || snap_bodies_[b] - slot_join_body_[s] >= (long long)st.itmax + 2) {

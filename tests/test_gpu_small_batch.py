@@ -71,3 +71,27 @@ def test_batch_same_bits_as_launches(cuda, precision):
     b2, r2 = _launched(solve)
     assert r1 == r2
     assert all(np.array_equal(u.x, v.x) for u, v in zip(b1, b2))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_expired_wait_ends_its_system_alone(cuda, precision):
+    """A barrier wait that runs out (a limit of no reads at all) ends that system with IER -15 in all
+    its blocks; a system of one block, which waits for none, is solved, and so is the next batch."""
+    one, many = S.conv_diff(4, 6, 3, seed=1), S.conv_diff(40, 64, 33, seed=5)
+
+    def solve():
+        batch = [one.copy(), many.copy()]
+        _, res = leq.batch_solve(batch, precision=precision)
+        return batch, [r.ier for r in res]
+
+    want, ier = solve()
+    assert ier == [0, 0]
+    assert leq.set_option("wait_polls", 0) == 0
+    try:
+        got, ier = solve()
+    finally:
+        assert leq.set_option("wait_polls", 2 ** 22) == 0
+    assert ier == [0, leq.IER_INCOMPLETE]
+    assert np.array_equal(got[0].x, want[0].x)
+    got, ier = solve()
+    assert ier == [0, 0] and all(np.array_equal(u.x, v.x) for u, v in zip(got, want))
