@@ -3943,23 +3943,20 @@ int prepare_line_kernel(int cmax, int *warps)
     if (wpb < 1) return 0;
     *warps = wpb;
     const int smem = wpb * per_warp;
-    // the limit is a property of the kernel, shared by every engine of the
-    // process (some on other threads): it only ever grows
+    // the limit is a property of the kernel in the current context, shared by the
+    // engines there (some on other threads): what is asked for only ever grows, and is
+    // asked for each time, since the context may be another one
     static std::mutex mu;
     static int granted = 0;
     constexpr int VMAX = sizeof(T) == 4 ? 4 : 2;  // widest instance
     {
         std::lock_guard<std::mutex> lk(mu);
-        if (smem > granted) {
-            if (cudaFuncSetAttribute(k_jline<T, VMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-                    cudaSuccess ||
-                cudaFuncSetAttribute(k_jline<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-                    cudaSuccess ||
-                cudaFuncSetAttribute(k_jline<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
-                    cudaSuccess)
-                return 0;
-            granted = smem;
-        }
+        const int ask = std::max(smem, granted);
+        if (cudaFuncSetAttribute(k_jline<T, VMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, ask) != cudaSuccess ||
+            cudaFuncSetAttribute(k_jline<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, ask) != cudaSuccess ||
+            cudaFuncSetAttribute(k_jline<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ask) != cudaSuccess)
+            return 0;
+        granted = ask;
     }
     int nb = 0, nb1 = 0, nb2 = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_jline<T, VMAX>, wpb * 32, smem) != cudaSuccess ||
@@ -4093,8 +4090,9 @@ template <typename T, bool MIXED>
 bool iterate_fits(const IterArgs &a)
 {
     constexpr int MOST = 180 * 1024;  // beside the static 16 KB
-    static const bool ready = cudaFuncSetAttribute(k_iterate<T, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   MOST) == cudaSuccess;
+    // asked for each time: the attribute belongs to the current context
+    const bool ready = cudaFuncSetAttribute(k_iterate<T, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST) ==
+                       cudaSuccess;
     cudaGetLastError();
     return ready && iterate_smem<T>(a) <= MOST;
 }
