@@ -185,7 +185,8 @@ const char *mfixgpu_last_error(void);
  *                    returns IER -15 (default 2^22, a second or two; 0..1e9)
  *   "time_kernels"   1: time every J-line sweep launch with CUDA events (no graph replay)
  *   "autotune"       1 (default): lanes per J-line picked by measurement for the new line lengths of a
- *                    solve or batch (one lanes-per-line value timed on all their lines at once)
+ *                    solve or batch (one lanes-per-line value timed on all their lines at once), where
+ *                    the length alone does not decide (lines that a warp's registers hold in one pass)
  *   "line_lanes"     0 (default) automatic, else lanes per J-line (1..32, rounded down to a power of two)
  * Returns 0, or MFIXGPU_ERR_ARGS for an unknown name. */
 int mfixgpu_set_option(const char *name, double value);
@@ -193,7 +194,9 @@ double mfixgpu_get_option(const char *name);
 
 /* Autotuner of the J-line kernel (no reference counterpart): its choices,
  * keyed by precision and line length, are read from and written to the JSON
- * file at `path` (NULL or "" keeps them in memory only). */
+ * file at `path` (NULL or "" keeps them in memory only).  Entries of lengths
+ * whose shape is decided without a measurement are written for information and
+ * not read. */
 int mfixgpu_autotune_cache(const char *path);
 /* Copies up to max_entries (element bytes, line length, lanes per line) triples
  * into out[3*i..3*i+2]; returns the number of entries recorded. */

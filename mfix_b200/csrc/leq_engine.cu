@@ -526,16 +526,49 @@ static void set_shape(SysDev &d, int elem, int shape)
     d.line_kind = g == 1 ? LK_THREAD : d.line_np ? LK_REG : LK_WARP;
 }
 
-// Lanes per J-line of a system (jmax2 set): a forced value, the autotuner's
-// choice for (precision, line length), or the default: the smallest power of two
-// that leaves at most 12 rows per lane (at most 32 lanes), widened while the
-// lanes' registers cannot hold the line.
+// The fewest lanes at which k_jline_reg takes its fewest passes over a line of
+// length L (0: it does not serve L).
+static int reg_lanes(int L, int elem)
+{
+    const int np = reg_passes(L, elem, 32);
+    int g = REG_MIN_LANES;
+    while (np && reg_passes(L, elem, g) != np) g *= 2;
+    return np ? g : 0;
+}
+
+// Whether a line of length L takes k_jline_reg's shape without a timing.  The choice
+// is by precision and length alone, never by the batch, so that a system's bits and
+// its speed do not depend on what was solved with it or before it.  One pass, and
+// lanes that mostly hold a chunk; times of the register kernel over the best k_jline
+// shape, four launched half-sweeps of 6M cells / 60 iterations of k_iterate:
+//   FP32  L = 6..8 1.11..1.07 / 0.97..0.99; 10..14 1.03..1.01 / 0.90..0.86; 18..130
+//         0.94..0.99 / 0.85..0.92; 146 1.00 / 0.92; 173 1.02 / 0.92; 178..260 0.95..0.99 / 0.90
+//   FP64  at least 5/8 of the lanes' rows: 0.82..1.01 / 0.69..0.96; less, on more than
+//         four lanes (L = 36, 68, 76): 1.05..1.06 / 1.07..1.15
+// Two passes (FP64 L = 132..178 1.02..1.22, 194..258 0.79..1.00; FP32 260..514
+// 0.99..1.03) are timed: k_iterate does not serve them.
+static bool reg_by_rule(int L, int elem)
+{
+    if (reg_passes(L, elem, 32) != 1) return false;
+    if (elem == 4) return L > 8;
+    const int g = reg_lanes(L, elem);
+    return g == REG_MIN_LANES || 8 * L >= 5 * g * (32 / elem);
+}
+
+// Lanes per J-line of a system (jmax2 set): a forced value, the register kernel's
+// shape by rule, the autotuner's choice for (precision, line length), or the default:
+// the smallest power of two that leaves at most 12 rows per lane (at most 32 lanes),
+// widened while the lanes' registers cannot hold the line.
 void Engine::shape_for(SysDev &d, int elem, int forced)
 {
     if (forced > 0) {
         int g = 1;
         while (g * 2 <= std::min(forced, 32)) g *= 2;
         set_shape(d, elem, g);
+        return;
+    }
+    if (reg_by_rule(d.jmax2, elem)) {
+        set_shape(d, elem, reg_lanes(d.jmax2, elem));
         return;
     }
     {
@@ -553,11 +586,12 @@ void Engine::shape_for(SysDev &d, int elem, int forced)
     set_shape(d, elem, g);
 }
 
-// The autotuner: for the line lengths of the batch without a recorded choice, time
-// a red/black pass of the J-line kernel over all their lines at once (the other
-// systems' line work masked out) for each lanes-per-line value g and each of the
-// two kernels, each length taking the shape nearest to it that can hold its lines
-// (shape_of below), and keep the fastest for all of them.  Timing the whole mix at
+// The autotuner: for the line lengths of the batch that have neither a rule nor a
+// recorded choice, time a red/black pass of the J-line kernels over all their lines at
+// once (the other systems' line work masked out) for each lanes-per-line value g of
+// k_jline, each length taking the shape nearest to it that can hold its lines (shape_of
+// below), lengths that k_jline_reg serves in two passes with either kernel, and keep
+// the fastest for all of them.  Timing the whole mix at
 // once ranks the shapes as the batch runs them: timing each length alone, on its
 // few systems, left a 512-system FP64 batch 10% slower than one shape for every
 // line.
@@ -569,6 +603,7 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
         const int L = h_sys_[s].jmax2;
         {
             std::lock_guard<std::mutex> lk(tunes().mu);
+            if (reg_by_rule(L, elem)) tunes().lanes[std::make_pair(elem, L)] = reg_lanes(L, elem);  // for the table
             if (tunes().lanes.count(std::make_pair(elem, L))) continue;
         }
         if (std::find(todo.begin(), todo.end(), L) == todo.end()) todo.push_back(L);
@@ -585,28 +620,24 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
         w[q].write_old = 1;
         w[q].gate = G_ANY;
     }
-    // the shape of length L under the candidate (g, staged): the smallest power of
-    // two at or above g at which k_jline_reg takes its fewest passes, or, staged or for
-    // a line that kernel does not serve, that leaves a lane at most MAX_TUNED_ROWS
-    // rows; for a line too long for that, 32 while its staging stays within 48 KB per
-    // warp, else none (0: the candidate is skipped)
+    // the shape of length L under the candidate (g, staged): k_jline_reg's for two
+    // passes unless staged, else the smallest power of two at or above g that leaves a
+    // lane at most MAX_TUNED_ROWS rows; for a line too long for that, 32 while its
+    // staging stays within 48 KB per warp, else none (0: the candidate is skipped)
     auto shape_of = [&](int L, int g, bool staged) {
-        if (g == 1) return 1;
         const int np = reg_passes(L, elem, 32);  // 0: k_jline_reg does not serve L
-        for (int h = g; h <= 32; h *= 2) {
-            if (np > 0 && !staged) {
-                if (reg_passes(L, elem, h) == np) return h;
-            } else if (rows_for(L, h) <= MAX_TUNED_ROWS &&
-                       (size_t)kernel_smem_line_bytes(rows_for(L, h), elem) <= 48 * 1024) {
+        if (np == 2 && !staged) return reg_lanes(L, elem);
+        if (g == 1) return 1;
+        for (int h = g; h <= 32; h *= 2)
+            if (rows_for(L, h) <= MAX_TUNED_ROWS && (size_t)kernel_smem_line_bytes(rows_for(L, h), elem) <= 48 * 1024)
                 return np > 0 ? h | LINE_STAGED : h;
-            }
-        }
         return (size_t)kernel_smem_line_bytes(rows_for(L, 32), elem) <= 48 * 1024 ? (np > 0 ? 32 | LINE_STAGED : 32) : 0;
     };
-    bool any_reg = false, any_long = false, one_pass = true;
+    bool any_two = false, all_two = true, any_long = false;
     for (int L : todo) {
-        one_pass = one_pass && reg_passes(L, elem, 32) == 1;
-        any_reg = any_reg || reg_passes(L, elem, 32) > 0;
+        const bool two = reg_passes(L, elem, 32) == 2;
+        any_two = any_two || two;
+        all_two = all_two && two;
         any_long = any_long || L > 32;
     }
     // the timing events and the tuning mask are released on every way out
@@ -627,24 +658,21 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
     int best_g = 0;
     bool best_staged = false;
     float best_ms = 1e30f;
-    // the register kernel's one shape first (the fewest lanes that hold a line in its
-    // fewest passes: more lanes idle), then k_jline at every width, which has to be 5%
-    // faster where the register kernel serves the batch (62-63 us against 66 for four
-    // FP32 half-sweeps of 145x173x100 cells, 336 against 290 of 258^3): k_iterate, which
-    // has few warps, prefers the shape with the most lines a warp.  One lane per line
-    // for short lines only (at 66 cells it takes nine times the best width's time).
-    // A batch small enough for k_iterate launches sweeps of 3-4 us, which all time alike
-    // (26 to 35 us for four at 66^3 to 80^3 cells, the choice a matter of chance): there the
-    // register kernel is taken without a timing where it serves every line in one pass
-    // (60 iterations at 74^3: FP32 12.9 ms with k_jline's shape, 9.6 with this one, FP64
-    // 6.5 and 5.4), and elsewhere a wider shape has to be 5% faster (FP64 at 65^3: 5.1 ms
-    // with 16 lanes, 6.1 with 32).
+    // Lengths of two passes: the register kernel first, k_jline has to be 5% faster
+    // (336 us against 290 for four FP32 half-sweeps of 258^3 cells with the earlier
+    // tuner's shape).  A batch small enough for k_iterate, which serves k_jline's lines
+    // and not two passes, takes k_jline there (60 iterations of 0.5M FP64 cells, L = 132
+    // to 258: 5.8 to 7.6 ms, with the launches of two passes 7.6 to 8.5); its launched
+    // sweeps of 3-4 us all time alike, so a wider shape has to be 5% faster (FP64 at
+    // 65^3: 5.1 ms with 16 lanes, 6.1 with 32).  One lane per line for short lines of
+    // larger batches only (at 66 cells it takes nine times the best width's time, and
+    // k_iterate does not serve it).
     const bool small = view_.ntiles <= sms_;
-    const int cand_end = small && one_pass ? 0 : 6;
-    for (int cand = any_reg ? -1 : any_long ? 1 : 0; cand < cand_end; ++cand) {
-        if (any_reg && cand == 0) continue;
-        const int g = cand < 0 ? 2 : 1 << cand;
-        const bool staged = cand > 0 && any_reg;
+    for (int cand = any_two && !small ? 0 : 6; cand < 12; ++cand) {
+        const int g = 1 << cand % 6;
+        const bool staged = cand >= 6;
+        if (all_two && !staged && cand > 0) continue;  // one shape
+        if (g == 1 && (any_long || small) && (staged || !all_two)) continue;
         bool fits = true;
         for (int L : todo) fits = fits && shape_of(L, g, staged) > 0;
         if (!fits) continue;
@@ -694,9 +722,9 @@ void Engine::load_tune_cache(const std::string &path)
     int elem, L, G;
     char buf[256];
     while (std::fgets(buf, sizeof buf, f)) {
-        int staged = 0;  // absent in files of choices between widths alone
+        int staged = 1;  // absent in files of choices among k_jline's widths alone
         if (std::sscanf(buf, " {\"elem\": %d, \"L\": %d, \"lanes\": %d, \"staged\": %d}", &elem, &L, &G, &staged) >= 3 &&
-            G >= 1 && G <= 32)
+            G >= 1 && G <= 32 && !reg_by_rule(L, elem))
             tunes().lanes[std::make_pair(elem, L)] = G | (staged ? LINE_STAGED : 0);
     }
     std::fclose(f);

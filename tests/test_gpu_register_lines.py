@@ -48,6 +48,42 @@ def test_solve_line_lengths(cuda, precision, jmax, lanes):
     assert np.linalg.norm(r) <= 1.01e-8 * np.linalg.norm(w.b)
 
 
+def _solved_with(tmp_path, s, precision, entry):
+    """The solution after the choices file `entry` (None: no file) was read."""
+    if entry is not None:
+        path = tmp_path / "choices.json"
+        path.write_text("[\n  {%s}\n]\n" % entry)
+        assert leq.autotune_cache(str(path)) == 0
+    w = s.copy()
+    try:
+        rc, res = leq.batch_solve([w], precision=precision)
+    finally:
+        leq.autotune_cache(None)
+    assert rc == 0 and res[0].ier == 0
+    return w.x
+
+
+@pytest.mark.parametrize("precision,jmax", [(1, 74), (1, 171), (0, 98)])
+def test_one_pass_lines_keep_their_shape(cuda, tmp_path, precision, jmax):
+    """A length that the register kernel serves in one pass has one shape, whatever was chosen before
+    (another batch size, another process): the same bits."""
+    s = S.conv_diff(9, jmax, 7, seed=jmax)
+    elem, L = (4 if precision else 8), jmax + 2
+    want = _solved_with(tmp_path, s, precision, None)
+    for lanes in (8, 16):
+        entry = f'"elem": {elem}, "L": {L}, "lanes": {lanes}, "staged": 1'
+        assert np.array_equal(_solved_with(tmp_path, s, precision, entry), want)
+
+
+def test_choices_without_a_kernel_are_of_k_jline(cuda, tmp_path):
+    """Files from before k_jline_reg name no kernel: their choices were timed on k_jline."""
+    s = S.conv_diff(9, 198, 7, seed=4)
+    entry = '"elem": 8, "L": 200, "lanes": 32'
+    old = _solved_with(tmp_path, s, 0, entry)
+    assert np.array_equal(old, _solved_with(tmp_path, s, 0, entry + ', "staged": 1'))
+    assert not np.array_equal(old, _solved_with(tmp_path, s, 0, entry + ', "staged": 0'))
+
+
 def test_batch_of_mixed_parities_equals_alone(cuda):
     """FP64 systems of even and odd JMAX2 in one batch (two line kernels): each as alone."""
     sysm = [S.conv_diff(9, j, 7, seed=j) for j in (20, 21, 62, 63, 128, 131, 10)]
