@@ -1798,7 +1798,8 @@ __device__ __forceinline__ void xr_tile(const SysDev &d, const SysState &st, int
         if (!MIXED && (cnt & 1) && threadIdx.x == 0) x[cnt - 1] = x[cnt - 1] + alpha * (X_T)ph[cnt - 1];
     } else {
         const X_T omega = (X_T)st.omega;
-        const X_T wz = defl ? (X_T)(st.alpha * st.defl_cp + st.omega * st.defl_cs) : X_T(0);
+        // both products' roundings stated: this tile is inlined into two kernels
+        const X_T wz = defl ? (X_T)__fma_rn(st.omega, st.defl_cs, __dmul_rn(st.alpha, st.defl_cp)) : X_T(0);
         const T omega_t = (T)st.omega;
         const T *__restrict__ sh = vec<T>(d, sh_id) + c0;
         const T *__restrict__ s = vec<T>(d, V_S) + c0;
@@ -2352,21 +2353,18 @@ __device__ __forceinline__ RowsV<T, VW> ldv(const T *p)
     return *reinterpret_cast<const RowsV<T, VW> *>(p);
 }
 
-// c - a*b, a*b + c and a*b for the J-line sweeps: in FP32 with every rounding
-// stated (so that the register-staged and the bulk-staged kernels give the same
-// bits), in FP64 as written.
-template <typename T>
-__device__ __forceinline__ T fnms(T a, T b, T c) { return c - a * b; }
-template <>
-__device__ __forceinline__ float fnms<float>(float a, float b, float c) { return __fmaf_rn(-a, b, c); }
-template <typename T>
-__device__ __forceinline__ T fma_t(T a, T b, T c) { return a * b + c; }
-template <>
-__device__ __forceinline__ float fma_t<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-template <typename T>
-__device__ __forceinline__ T mul_t(T a, T b) { return a * b; }
-template <>
-__device__ __forceinline__ float mul_t<float>(float a, float b) { return __fmul_rn(a, b); }
+// c - a*b, a*b + c and a*b for the J-line sweeps, with every rounding stated: the line
+// solves are inlined into several kernels that have to give the same bits (launched or
+// in k_iterate), and in r*y - q*x a compiler may fuse either product.
+__device__ __forceinline__ float fnms(float a, float b, float c) { return __fmaf_rn(-a, b, c); }
+__device__ __forceinline__ double fnms(double a, double b, double c) { return __fma_rn(-a, b, c); }
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_t(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_t(double a, double b) { return __dmul_rn(a, b); }
+// r*y - q*x of k_jline's second recurrence.
+__device__ __forceinline__ float back_t(float r, float y, float q, float x) { return __fmaf_rn(-q, x, __fmul_rn(r, y)); }
+__device__ __forceinline__ double back_t(double r, double y, double q, double x) { return __fma_rn(r, y, -__dmul_rn(q, x)); }
 
 // The two recurrences of a factored line, y_r = f_r - l_r y_{r-1} and
 // x_r = r_r y_r - q_r x_{r+1}, on shared-memory rows: lane gl of the line's G
@@ -2404,7 +2402,7 @@ __device__ __forceinline__ void line_recurrences(T *f, const T *fl, const T *fr,
 #pragma unroll 4
     for (int t = c - 1; t >= 0; --t) {
         const T qt = cq[t];
-        mb = fnms(qt, mb, mul_t(cr[t], cf[t]));
+        mb = back_t(cr[t], cf[t], qt, mb);
         ma = -qt * ma;
     }
     for (int dl = 1; dl < G; dl <<= 1) {
@@ -2418,7 +2416,7 @@ __device__ __forceinline__ void line_recurrences(T *f, const T *fl, const T *fr,
     if (gl == G - 1) xv = T(0);
 #pragma unroll 4
     for (int t = c - 1; t >= 0; --t) {
-        xv = fnms(cq[t], xv, mul_t(cr[t], cf[t]));
+        xv = back_t(cr[t], cf[t], cq[t], xv);
         cf[t] = xv;
     }
 }
