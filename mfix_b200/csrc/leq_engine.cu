@@ -709,6 +709,10 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
                 set_shape(h_sys_[s], elem, g);
     }
     (void)opt;
+    // the timed sweeps are none of the solve's: their flagged lines leave its counts
+    static_assert(offsetof(SysState, line_fallbacks) == offsetof(SysState, line_skips) + sizeof(int), "adjacent counts");
+    CK(cudaMemset2DAsync(reinterpret_cast<char *>(d_st_) + offsetof(SysState, line_skips), sizeof(SysState), 0,
+                         2 * sizeof(int), (size_t)nsys_, stream_));
     save_tune_cache();
     return configure_lines(elem);
 }

@@ -48,6 +48,75 @@ def test_solve_line_lengths(cuda, precision, jmax, lanes):
     assert np.linalg.norm(r) <= 1.01e-8 * np.linalg.norm(w.b)
 
 
+def _flag_lines(s, seed):
+    """Five interior J-lines with one diagonal shrunk a hundredfold (DGTSV interchanges rows there) and
+    one without a tridiagonal (INFO != 0: left as it was); the system still converges."""
+    rng = np.random.default_rng(seed)
+    lines = [(i + k * s.imax2) * s.jmax2 for i in range(1, s.imax2 - 1) for k in range(1, s.kmax2 - 1)]
+    for base in rng.choice(lines, size=5, replace=False):
+        s.a[3, base + int(rng.integers(2, s.jmax2 - 2))] *= 0.01
+    base = lines[len(lines) // 2]
+    s.a[np.ix_([1, 3, 5], range(base + 1, base + s.jmax2 - 1))] = 0.0
+    return base
+
+
+@pytest.mark.parametrize("jmax", [14, 62, 128, 190])  # 4, 16 and 32 lanes, half a chunk, two passes
+def test_msolve_flagged_lines(cuda, jmax):
+    """Lines that the register kernel hands to DGTSV.  The oracle's result moves by 1.2e-15 at most
+    when each entry of A moves by an ulp; 1e-12 as for the lines without interchanges."""
+    s = S.conv_diff(7, jmax, 6, seed=jmax)
+    oracle.scale(s)
+    base = _flag_lines(s, jmax)
+    b = np.random.default_rng(4).standard_normal(s.n)
+    _, want, skips = oracle.msolve(s, b, "RSRS", "LINE")
+    assert skips > 0
+    da, db = cuda.from_numpy(s.a).to("cuda"), cuda.from_numpy(b).to("cuda")
+    x = cuda.zeros(s.n, dtype=cuda.float64, device="cuda")
+    cuda.cuda.synchronize()
+    g = leq.geom(s.imax2, s.jmax2, s.kmax2, s.do_k)
+    assert leq.leq_msolve(g, db.data_ptr(), da.data_ptr(), x.data_ptr(), "RSRS", "LINE") == 0
+    got = x.cpu().numpy()
+    assert np.array_equal(got[base:base + s.jmax2], b[base:base + s.jmax2])
+    assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("jmax", [14, 30, 66, 258])
+def test_solve_flagged_lines(cuda, precision, jmax):
+    """The same in whole solves, in k_iterate and launched (use_graph 0): equal bits, TOL met."""
+    s = S.conv_diff(9, jmax, 8, seed=jmax, tol=1e-8)
+    _flag_lines(s, jmax)
+    out = []
+    for graph in (1, 0):
+        w = s.copy()
+        assert leq.set_option("precision", precision) == 0 and leq.set_option("use_graph", graph) == 0
+        try:
+            assert leq.solve_system(w) == 0
+        finally:
+            leq.set_option("precision", 0)
+            leq.set_option("use_graph", 1)
+        st = leq.last_stats()
+        assert st["fp64_fallback"] == 0 and st["line_fallbacks"] > st["line_skips"] > 0
+        out.append((w.x, st["iterations"], st["line_fallbacks"], st["line_skips"]))
+    assert np.array_equal(out[0][0], out[1][0]) and out[0][1:] == out[1][1:]
+    r = w.b - S.matvec_np(w.imax2, w.jmax2, w.kmax2, w.do_k, w.a, w.x)
+    assert np.linalg.norm(r) <= 1.01e-8 * np.linalg.norm(w.b)
+
+
+def test_timed_sweeps_leave_the_counts(cuda):
+    """The first solve of a line length times the line kernels; those sweeps' flagged lines are not the
+    solve's.  JMAX2 = 87 (odd, FP64: a timed length) occurs in no other test."""
+    s = S.conv_diff(9, 85, 8, seed=5, tol=1e-8)
+    _flag_lines(s, 5)
+    counts = []
+    for _ in range(2):
+        w = s.copy()
+        assert leq.solve_system(w) == 0
+        st = leq.last_stats()
+        counts.append((st["line_skips"], st["line_fallbacks"]))
+    assert counts[0] == counts[1] and counts[0][0] > 0
+
+
 def _solved_with(tmp_path, s, precision, entry):
     """The solution after the choices file `entry` (None: no file) was read."""
     if entry is not None:
