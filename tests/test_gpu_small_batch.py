@@ -25,7 +25,7 @@ CASES = {
     "odd_2d": lambda: S.conv_diff(61, 47, 1, seed=3, do_k=False),
     "odd_3d": lambda: S.conv_diff(19, 25, 17, seed=4),
     "even_3d": lambda: S.conv_diff(40, 64, 33, seed=5),
-    "most_tiles": lambda: S.conv_diff(80, 66, 94, seed=6),  # 142 tiles of the 148 that fit
+    "most_tiles": lambda: S.conv_diff(89, 70, 90, seed=6),  # 148 tiles: one per SM
     "capped": lambda: S.conv_diff(24, 30, 22, seed=7, itmax=5, tol=1e-10),
     "deflated": lambda: S.pressure_scaled(24, 30, 22, seed=8, tol=1e-6),
     "cyclic": lambda: S.conv_diff_cyclic(12, 16, 10, seed=9, cyc=5),
@@ -46,13 +46,22 @@ def test_same_bits_as_launches(cuda, case, precision):
             leq.set_option("precision", 0)
         st = leq.last_stats()
         return ier, w, {k: st[k] for k in ("iterations", "outer_steps", "exit_kind", "rnorm", "rnorm0", "deflated",
-                                           "fp64_fallback", "line_skips", "line_fallbacks")}
+                                           "fp64_fallback", "line_skips", "line_fallbacks")}, st["kernel_launches"]
 
     solve()  # the line shapes are tuned now
-    i1, w1, s1 = solve()
-    i2, w2, s2 = _launched(solve)
+    i1, w1, s1, n1 = solve()
+    i2, w2, s2, n2 = _launched(solve)
     assert i1 == i2 and s1 == s2
+    assert n2 - n1 > 8 * s1["iterations"]  # k_iterate took the iterations of the first solve
     assert np.array_equal(w1.x, w2.x) and np.array_equal(w1.a, w2.a) and np.array_equal(w1.b, w2.b)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_one_tile_too_many_is_launched(cuda, precision):
+    """149 tiles on 148 SMs: every kernel of an iteration is launched by itself."""
+    s = S.conv_diff(90, 70, 90, seed=6, itmax=5, tol=1e-30)
+    rc, res = leq.batch_solve([s], precision=precision)
+    assert rc == 0 and leq.last_stats()["kernel_launches"] > 8 * 5
 
 
 @pytest.mark.parametrize("precision", [0, 1])
