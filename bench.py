@@ -175,6 +175,16 @@ def ncu_traffic(kernel_file: str):
     return None
 
 
+def line_kernel(elem: int, line_length: int, w: str):
+    """The J-line kernel that serves the line length now, and the DRAM bytes per launch of a capture of it."""
+    from mfix_b200 import leq
+
+    k = leq.line_kernel(elem, line_length)
+    name, t = leq.LINE_KERNELS[k], "float" if elem == 4 else "double"
+    full = f"{name}<{t}, {k}>" if name == "k_jline_reg" else f"{name}<{t}>"
+    return f"{full} (LINE preconditioner half-sweep)", ncu_traffic(f"{name[2:]}_f{8 * elem}_{w}.md")
+
+
 class ClockSampler:
     """nvidia-smi clocks / throttle reasons sampled every 200 ms during the timed region."""
 
@@ -646,8 +656,8 @@ def run_ours(args) -> None:
     jl_work = min(work_m["jline"], jl_n)  # launches that did work (the rest returned at once)
     avg_launch_s = (jl_ms / 1e3) / max(jl_work, 1)
     achieved = alg_bytes_launch / avg_launch_s / 1e9
-    traffic = ncu_traffic(f"jline_f32_{w}.md")
-    roof = {"kernel": "k_jline_reg<float, NP> (LINE preconditioner half-sweep)", "bound": "hbm", "achieved": achieved,
+    kernel, traffic = line_kernel(4, sys0.jmax2, w)
+    roof = {"kernel": kernel, "bound": "hbm", "achieved": achieved,
             "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_kind": f"{peak_kind} (MEASURED_PEAKS hbm_gbs)",
             "alg_bytes_per_launch": alg_bytes_launch, "avg_launch_ms": avg_launch_s * 1e3, "launches": jl_n,
             "work_launches": jl_work, "traffic": traffic}
@@ -805,6 +815,7 @@ def run_cg_bench(args) -> None:
         kernels[names[k]] = {"ms": round(ms, 3), "launches": nl, "work_launches": nw,
                              "us_per_launch": round(1e3 * ms / max(nw, 1), 2), "gbs": round(gbs, 1),
                              "frac": round(gbs / peak, 3)}
+    kernel, traffic = line_kernel(8, sys0.jmax2, w)
     line = {
         "metric": "solves/s", "value": value, "unit": "solves/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": tot_dev / args.steps, "higher_is_better": True, "scaling": "weak",
@@ -812,10 +823,10 @@ def run_cg_bench(args) -> None:
         "config": {"workload": w, "grid": list(WORKLOADS[w]["dims"]), "cells": n, "method": 5, "pc": "LINE",
                    "sweep": "RSRS", "tol": sys0.tol, "itmax": sys0.itmax,
                    "l2_policy": "inputs larger than L2 (A_M 7*8*cells bytes), no flush needed"},
-        "roofline": {"kernel": "k_jline_reg<double, NP> (LINE preconditioner half-sweep)", "bound": "hbm",
+        "roofline": {"kernel": kernel, "bound": "hbm",
                      "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_kind": peak_kind, "alg_bytes_per_launch": alg_launch, "avg_launch_ms": avg_s * 1e3,
-                     "launches": jl_n, "work_launches": jl_work, "traffic": ncu_traffic(f"jline_f64_{w}.md")},
+                     "launches": jl_n, "work_launches": jl_work, "traffic": traffic},
         "e2e": {"value": e2e_value, "unit": "solves/s", "h2d_bytes_per_step": 9 * 8 * n,
                 "d2h_bytes_per_step": 9 * 8 * n, "entry": "mfixgpu_solve_lin_eq_ METHOD 5 (pinned host arrays)"},
         "gpu_launches": int(launches),

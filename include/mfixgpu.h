@@ -201,6 +201,11 @@ int mfixgpu_autotune_cache(const char *path);
 /* Copies up to max_entries (element bytes, line length, lanes per line) triples
  * into out[3*i..3*i+2]; returns the number of entries recorded. */
 int mfixgpu_autotune_table(int *out, int max_entries);
+/* The kernel that sweeps J-lines of line_length cells in arrays of element_bytes
+ * (4: the mixed form, 8: FP64) at the present options and choices: 0 k_jline (rows
+ * in shared memory), 1 or 2 k_jline_reg (rows in registers, passes over a line),
+ * 3 k_jline_thread (one lane per line).  Needs no device. */
+int mfixgpu_line_kernel(int element_bytes, int line_length);
 
 /* Releases device memory and the per-device engine. */
 void mfixgpu_finalize(void);

@@ -757,6 +757,17 @@ int mfixgpu_autotune_cache(const char *path)
     return 0;
 }
 
+int mfixgpu_line_kernel(int element_bytes, int line_length)
+{
+    if ((element_bytes != 4 && element_bytes != 8) || line_length < 1) return MFIXGPU_ERR_ARGS;
+    Global &g = G();
+    std::lock_guard<std::mutex> lk(g.mu);
+    SysDev d{};
+    d.jmax2 = line_length;
+    Engine::shape_for(d, element_bytes, g.opt.line_lanes);
+    return d.line_kind == LK_THREAD ? 3 : d.line_kind == LK_REG ? d.line_np : 0;
+}
+
 int mfixgpu_autotune_table(int *out, int max_entries)
 {
     Global &g = G();

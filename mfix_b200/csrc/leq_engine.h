@@ -192,6 +192,9 @@ public:
     int msolve(const SystemSpec &g, const double *a, const double *b, double *var, int pc, const char sweep[4]);
     int dot(const double *x, const double *y, int64_t n, double *out_host);
 
+    // the line shape of a system whose jmax2 is set; forced > 0: lanes per line
+    static void shape_for(SysDev &d, int elem, int forced);
+
 private:
     int run_batch(const std::vector<SystemSpec> &specs, const SolveOptions &opt, std::vector<SolveResult> &out);
     int run_batch_live(const std::vector<SystemSpec> &specs, const SolveOptions &opt, std::vector<SolveResult> &out);
@@ -205,7 +208,6 @@ private:
     int bind_lists();
     int configure_lines(int elem, int only_L = 0);
     std::vector<int> tune_lengths_;  // configure_lines(elem, -1): the line lengths being tuned
-    void shape_for(SysDev &d, int elem, int forced);
     int autotune_lines(const SolveOptions &opt, int elem);
     void save_tune_cache();
 

@@ -203,6 +203,8 @@ def _declare(L: C.CDLL) -> None:
     L.mfixgpu_autotune_cache.restype = C.c_int
     L.mfixgpu_autotune_table.argtypes = [C.POINTER(C.c_int), C.c_int]
     L.mfixgpu_autotune_table.restype = C.c_int
+    L.mfixgpu_line_kernel.argtypes = [C.c_int, C.c_int]
+    L.mfixgpu_line_kernel.restype = C.c_int
 
 
 def _ptr(a: np.ndarray) -> int:
@@ -315,6 +317,15 @@ def autotune_table() -> list[tuple[int, int, int]]:
     buf = (C.c_int * max(3 * n, 3))()
     n = lib().mfixgpu_autotune_table(buf, n)
     return [(buf[3 * q], buf[3 * q + 1], buf[3 * q + 2]) for q in range(n)]
+
+
+LINE_KERNELS = ("k_jline", "k_jline_reg", "k_jline_reg", "k_jline_thread")
+
+
+def line_kernel(element_bytes: int, line_length: int) -> int:
+    """Which J-line kernel serves lines of that length now: an index of LINE_KERNELS (1 and 2 are
+    k_jline_reg's passes over a line)."""
+    return lib().mfixgpu_line_kernel(element_bytes, line_length)
 
 
 def geom(imax2: int, jmax2: int, kmax2: int, do_k: int, cyclic: int = 0) -> Geom:

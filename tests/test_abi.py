@@ -47,6 +47,22 @@ def test_geometry_validation():
     assert leq.init_geometry(0, 5, 6, 1, 0, 0) == leq.IER_ARGS
 
 
+def test_line_kernel_by_precision_and_length():
+    """One pass in registers: by rule, whatever was solved before; odd FP64 and long lines never."""
+    for L in (9, 18, 66, 173, 260):
+        assert leq.line_kernel(4, L) == 1
+    for L in (6, 18, 20, 50, 66, 80, 130):
+        assert leq.line_kernel(8, L) == 1
+    for elem, L in ((8, 67), (8, 131), (4, 600), (8, 300)):
+        assert leq.LINE_KERNELS[leq.line_kernel(elem, L)] == "k_jline"
+    assert leq.line_kernel(2, 10) == leq.line_kernel(4, 0) == leq.IER_ARGS
+    assert leq.set_option("line_lanes", 1) == 0
+    try:
+        assert leq.LINE_KERNELS[leq.line_kernel(4, 66)] == "k_jline_thread"
+    finally:
+        leq.set_option("line_lanes", 0)
+
+
 def test_options_roundtrip():
     assert leq.set_option("precision", 1) == 0 and leq.get_option("precision") == 1
     assert leq.set_option("precision", 0) == 0
