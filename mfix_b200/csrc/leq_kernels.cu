@@ -8,12 +8,15 @@
 // The result is independent of which block finishes last and of what else is in
 // the batch, so a system gives bit-identical results alone and in a mix.
 //
-// J-line kernels give each warp one or more whole lines (G lanes per line).
-// Each lane eliminates a chunk of c consecutive rows to an interface form, the
-// 2G interface rows are solved by parallel cyclic reduction over shuffles, and
-// the interior rows are recovered in place.  Lines whose rows do not satisfy a
-// local dominance bound (under which DGTSV never interchanges rows) are solved
-// again by one lane with the exact pivoting DGTSV recurrence.
+// J-line kernels give each warp one or more whole lines (G lanes per line).  The
+// lines' tridiagonals are factored once per solve (k_line_factor), so a sweep runs two
+// linear recurrences down each line: a lane forms the affine map of its rows, a
+// shuffle scan composes the lanes' maps, and the lane runs its rows again from the
+// value that enters them.  k_jline_reg keeps the rows in registers, k_jline in shared
+// memory, k_jline_thread gives a lane a whole line.  Lines on which DGTSV interchanges
+// rows or meets a zero pivot (the factorization's own tests) are solved by one lane
+// with the exact pivoting DGTSV recurrence.  k_iterate runs whole iterations of a small
+// batch in one launch.
 #include <cfloat>
 #include <cstdio>
 #include <algorithm>
@@ -2362,7 +2365,8 @@ __device__ __forceinline__ float fma_t(float a, float b, float c) { return __fma
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float mul_t(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_t(double a, double b) { return __dmul_rn(a, b); }
-// r*y - q*x of k_jline's second recurrence.
+// r*y - q*x of k_jline's second recurrence, each precision with the product fused that
+// it has always fused.
 __device__ __forceinline__ float back_t(float r, float y, float q, float x) { return __fmaf_rn(-q, x, __fmul_rn(r, y)); }
 __device__ __forceinline__ double back_t(double r, double y, double q, double x) { return __fma_rn(r, y, -__dmul_rn(q, x)); }
 
@@ -2711,6 +2715,13 @@ __global__ void __launch_bounds__(128) k_jline_thread(BatchView b, WaveArgs w)
 // 73.2 us here; FP64 153.3 and 143.3 us.  Three blocks of four warps per SM (150
 // registers) keep the rows of twelve lines in flight per SM; four blocks spill and
 // take 302 us for four half-sweeps against 240 of the same loop without spills.
+//
+// FP32 pad rows (JMAX2 to the pitch) take part as rows with zero coefficients and
+// factors: they leave the line alone while the vectors' pads are finite (0 * pad).  The
+// setup zeroes the pads and later steps write zeros times the iteration's scalars
+// there; a scalar that overflows makes the cells themselves overflow in that iteration,
+// and with them the FP64 solution, whose residual then sends the system to the FP64 form
+// (fin_outer) before a pad counts.
 enum : int { LR_F = 0, LR_L, LR_R, LR_Q, LR_M0, LR_M1, LR_M2, LR_M3, LR_N };  // B, factors, A(-1), A(1), A(-3), A(3)
 
 // A warp's copy of what every line of the system it works on needs.

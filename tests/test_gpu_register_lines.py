@@ -117,6 +117,26 @@ def test_timed_sweeps_leave_the_counts(cuda):
     assert counts[0] == counts[1] and counts[0][0] > 0
 
 
+@pytest.mark.parametrize("scale", [1e36, 1e37, 1e38, 1e40])
+@pytest.mark.parametrize("graph", [0, 1])
+def test_fp32_overflow_is_no_answer(cuda, scale, graph):
+    """Right-hand sides whose iteration overflows FP32 (and leaves NaN in the padded lines' pads): the
+    FP64 form's verdict, not a wrong answer."""
+    s = S.conv_diff(9, 171, 7, seed=6, tol=1e-8)
+    s.b *= scale
+    assert leq.set_option("precision", 1) == 0 and leq.set_option("use_graph", graph) == 0
+    try:
+        w = s.copy()
+        assert leq.solve_system(w) == 0
+    finally:
+        leq.set_option("precision", 0)
+        leq.set_option("use_graph", 1)
+    if scale > 1e39:  # not even the right-hand side is an FP32 number
+        assert leq.last_stats()["fp64_fallback"] == 1
+    r = w.b - S.matvec_np(w.imax2, w.jmax2, w.kmax2, w.do_k, w.a, w.x)
+    assert np.linalg.norm(r) <= 1.01e-8 * np.linalg.norm(w.b)
+
+
 def _solved_with(tmp_path, s, precision, entry):
     """The solution after the choices file `entry` (None: no file) was read."""
     if entry is not None:
