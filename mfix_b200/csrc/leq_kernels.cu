@@ -1802,7 +1802,7 @@ __device__ __forceinline__ void xr_tile(const SysDev &d, const SysState &st, int
     } else {
         const X_T omega = (X_T)st.omega;
         // both products' roundings stated: this tile is inlined into two kernels
-        const X_T wz = defl ? (X_T)__fma_rn(st.omega, st.defl_cs, __dmul_rn(st.alpha, st.defl_cp)) : X_T(0);
+        const X_T wz = defl ? (X_T)__fma_rn(st.alpha, st.defl_cp, __dmul_rn(st.omega, st.defl_cs)) : X_T(0);
         const T omega_t = (T)st.omega;
         const T *__restrict__ sh = vec<T>(d, sh_id) + c0;
         const T *__restrict__ s = vec<T>(d, V_S) + c0;
