@@ -69,7 +69,12 @@ __device__ __forceinline__ uint32_t fdiv(uint32_t n, const FastDiv &f)
 // shared memory (k_jline) or keep them in registers (k_jline_reg), or one lane
 // runs a whole line (k_jline_thread).
 enum LineKind : int { LK_WARP = 0, LK_THREAD = 1, LK_REG = 2 };
-constexpr int REG_PASSES = 2;     // k_jline_reg: passes over a line at most
+// k_jline_reg: passes over a line at most.  FP32 lines of two passes (more than 260
+// cells) stay with k_jline: four half-sweeps of 6M cells take 0.99 to 1.03 times its
+// time there, and deflated mixed solves took 3 to 13% more iterations at each of five
+// sizes (JMAX2 = 302, 386; ten sets each) and were handed to FP64 more often (6 of 50
+// against 4, at 194 x 386 x 194 3 of 6 against 1 of 9).
+__host__ __device__ constexpr int reg_passes_max(int elem) { return elem == 4 ? 1 : 2; }
 constexpr int REG_MIN_LANES = 4;  // and lanes per line at least
 
 // One system of the batch.

@@ -495,7 +495,7 @@ static int reg_passes(int L, int elem, int G)
     if (G < REG_MIN_LANES || (elem == 8 && (L & 1))) return 0;
     const int chunk = G * 32 / elem, half = 16 / elem;
     const int np = std::max(1, (L - half + chunk - 1) / chunk);
-    return np <= REG_PASSES ? np : 0;
+    return np <= reg_passes_max(elem) ? np : 0;
 }
 
 // Most rows per lane the autotuner gives the shared-memory kernel, whose staging
@@ -545,8 +545,8 @@ static int reg_lanes(int L, int elem)
 //         0.94..0.99 / 0.85..0.92; 146 1.00 / 0.92; 173 1.02 / 0.92; 178..260 0.95..0.99 / 0.90
 //   FP64  at least 5/8 of the lanes' rows: 0.82..1.01 / 0.69..0.96; less, on more than
 //         four lanes (L = 36, 68, 76): 1.05..1.06 / 1.07..1.15
-// Two passes (FP64 L = 132..178 1.02..1.22, 194..258 0.79..1.00; FP32 260..514
-// 0.99..1.03) are timed: k_iterate does not serve them.
+// Two passes (FP64 L = 132..178 1.02..1.22, 194..258 0.79..1.00) are timed: k_iterate
+// does not serve them.
 static bool reg_by_rule(int L, int elem)
 {
     if (reg_passes(L, elem, 32) != 1) return false;
@@ -659,8 +659,7 @@ int Engine::autotune_lines(const SolveOptions &opt, int elem)
     bool best_staged = false;
     float best_ms = 1e30f;
     // Lengths of two passes: the register kernel first, k_jline has to be 5% faster
-    // (336 us against 290 for four FP32 half-sweeps of 258^3 cells with the earlier
-    // tuner's shape).  A batch small enough for k_iterate, which serves k_jline's lines
+    // (601 us against 570 for four FP64 half-sweeps of 258^3 cells).  A batch small enough for k_iterate, which serves k_jline's lines
     // and not two passes, takes k_jline there (60 iterations of 0.5M FP64 cells, L = 132
     // to 258: 5.8 to 7.6 ms, with the launches of two passes 7.6 to 8.5); its launched
     // sweeps of 3-4 us all time alike, so a wider shape has to be 5% faster (FP64 at

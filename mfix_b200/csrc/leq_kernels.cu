@@ -2710,9 +2710,10 @@ __global__ void __launch_bounds__(128) k_jline_thread(BatchView b, WaveArgs w)
 // accesses per chunk took 41.1 us per half-sweep on 129x147x122 cells against 33.8
 // of k_jline, which keeps those lines.)
 //
-// Bound by HBM: 258^3 cells, one half-sweep (20 / 40 bytes per cell): FP32 86.0 us
-// with k_jline's exchange through shared memory (1050 warp instructions a line),
-// 73.2 us here; FP64 153.3 and 143.3 us.  Three blocks of four warps per SM (150
+// Bound by load latency (at 194^3 in FP32 57-64% of a warp's cycles an instruction wait
+// for loads, DRAM at half its rate): 258^3 cells, one half-sweep (20 / 40 bytes per
+// cell): FP32 86.0 us with k_jline's exchange through shared memory (1050 warp
+// instructions a line), 73.2 us here; FP64 153.3 and 143.3 us.  Three blocks of four warps per SM (150
 // registers) keep the rows of twelve lines in flight per SM; four blocks spill and
 // take 302 us for four half-sweeps against 240 of the same loop without spills.
 //
@@ -4000,7 +4001,7 @@ static int occ(K kern, int threads = CELL_THREADS)
 template <typename T>
 int line_reg_occupancy(int np)
 {
-    static const int nb[2] = {occ(k_jline_reg<T, 1>, 128), occ(k_jline_reg<T, REG_PASSES>, 128)};
+    static const int nb[2] = {occ(k_jline_reg<T, 1>, 128), occ(k_jline_reg<T, reg_passes_max(sizeof(T))>, 128)};
     return nb[np <= 1 ? 0 : 1];
 }
 
@@ -4075,7 +4076,8 @@ cudaError_t launch_jline(const BatchView &b, const LaunchCfg &c, const WaveArgs 
     // their lines have even length
     if (c.line_thread) k_jline_thread<T><<<c.line_grid_thread, 128, 0, c.stream>>>(b, w);
     if (c.line_reg & 1) k_jline_reg<T, 1><<<c.line_grid_reg[0], 128, 0, c.stream>>>(b, w);
-    if (c.line_reg & 2) k_jline_reg<T, REG_PASSES><<<c.line_grid_reg[1], 128, 0, c.stream>>>(b, w);
+    if constexpr (reg_passes_max(sizeof(T)) > 1)
+        if (c.line_reg & 2) k_jline_reg<T, 2><<<c.line_grid_reg[1], 128, 0, c.stream>>>(b, w);
     if (c.line_warp) {
         const int smem = c.line_warps * kernel_smem_line_bytes(c.line_cmax, (int)sizeof(T));
         constexpr int VMAX = sizeof(T) == 4 ? 4 : 2;

@@ -53,7 +53,7 @@ def test_line_kernel_by_precision_and_length():
         assert leq.line_kernel(4, L) == 1
     for L in (6, 18, 20, 50, 66, 80, 130):
         assert leq.line_kernel(8, L) == 1
-    for elem, L in ((8, 67), (8, 131), (4, 600), (8, 300)):
+    for elem, L in ((8, 67), (8, 131), (4, 261), (4, 386), (4, 600), (8, 300)):
         assert leq.LINE_KERNELS[leq.line_kernel(elem, L)] == "k_jline"
     assert leq.line_kernel(2, 10) == leq.line_kernel(4, 0) == leq.IER_ARGS
     assert leq.set_option("line_lanes", 1) == 0
