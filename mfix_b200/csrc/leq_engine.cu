@@ -558,7 +558,10 @@ static bool reg_by_rule(int L, int elem)
 // Lanes per J-line of a system (jmax2 set): a forced value, the register kernel's
 // shape by rule, the autotuner's choice for (precision, line length), or the default:
 // the smallest power of two that leaves at most 12 rows per lane (at most 32 lanes),
-// widened while the lanes' registers cannot hold the line.
+// widened while the lanes' registers cannot hold the line.  FP64 lines of two passes
+// that k_jline holds with 11 rows on 16 lanes stay there: one msolve of 4M cells at
+// L = 132, 146, 160, 170, 176 takes 453, 515, 460, 554, 504 us with k_jline and 488, 525,
+// 485, 544, 518 with two passes; at 178, 194, 258 638, 584, 660 and 555, 572, 641.
 void Engine::shape_for(SysDev &d, int elem, int forced)
 {
     if (forced > 0) {
@@ -582,6 +585,10 @@ void Engine::shape_for(SysDev &d, int elem, int forced)
     int g = 1;
     while (g < 32 && g * 12 < d.jmax2) g *= 2;
     const int np = reg_passes(d.jmax2, elem, 32);
+    if (np == 2 && d.jmax2 <= 16 * 11) {
+        set_shape(d, elem, g | LINE_STAGED);
+        return;
+    }
     while (g > 1 && g < 32 && np && reg_passes(d.jmax2, elem, g) != np) g *= 2;
     set_shape(d, elem, g);
 }

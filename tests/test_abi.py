@@ -55,6 +55,10 @@ def test_line_kernel_by_precision_and_length():
         assert leq.line_kernel(8, L) == 1
     for elem, L in ((8, 67), (8, 131), (4, 261), (4, 386), (4, 600), (8, 300)):
         assert leq.LINE_KERNELS[leq.line_kernel(elem, L)] == "k_jline"
+    for L in (132, 160, 176):  # untimed: k_jline's 16 lanes are faster than two passes
+        assert leq.line_kernel(8, L) == 0
+    for L in (178, 194, 258):
+        assert leq.line_kernel(8, L) == 2
     assert leq.line_kernel(2, 10) == leq.line_kernel(4, 0) == leq.IER_ARGS
     assert leq.set_option("line_lanes", 1) == 0
     try:
