@@ -2749,11 +2749,12 @@ __device__ __forceinline__ void ld_rows(float *v, const char *p)
 {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
                  : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
-                 : "l"(p));
+                 : "l"(p)
+                 : "memory");
 }
 __device__ __forceinline__ void ld_rows(double *v, const char *p)
 {
-    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];\n" : "=d"(v[0]), "=d"(v[1]) : "l"(p));
+    asm volatile("ld.global.v2.f64 {%0, %1}, [%2];\n" : "=d"(v[0]), "=d"(v[1]) : "l"(p) : "memory");
 }
 __device__ __forceinline__ void st_rows(char *p, const float *v)
 {
