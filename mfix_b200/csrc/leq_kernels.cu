@@ -3941,6 +3941,9 @@ cudaError_t launch_p_update(const BatchView &b, const LaunchCfg &c)
 // Shared memory of one warp of the J-line kernel: right-hand side and the three factor rows.
 int kernel_smem_line_bytes(int cmax, int elem_bytes) { return 4 * 32 * cmax * elem_bytes; }
 
+// Dynamic shared memory that a kernel may use beside 16 KB of static without asking.
+constexpr int SMEM_UNASKED = 32 * 1024;
+
 // Picks the warps per block that fit the staging buffers, sets the shared-memory
 // attribute and returns the resident blocks per SM (0 when a line cannot fit).
 template <typename T>
@@ -3956,11 +3959,12 @@ int prepare_line_kernel(int cmax, int *warps)
     const int smem = wpb * per_warp;
     // the limit is a property of the kernel in the current context, shared by the
     // engines there (some on other threads): what is asked for only ever grows, and is
-    // asked for each time, since the context may be another one
+    // asked for each time, since the context may be another one, but not where the
+    // limit that every kernel has suffices
     static std::mutex mu;
     static int granted = 0;
     constexpr int VMAX = sizeof(T) == 4 ? 4 : 2;  // widest instance
-    {
+    if (smem > SMEM_UNASKED) {
         std::lock_guard<std::mutex> lk(mu);
         const int ask = std::max(smem, granted);
         if (cudaFuncSetAttribute(k_jline<T, VMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, ask) != cudaSuccess ||
@@ -4102,11 +4106,13 @@ template <typename T, bool MIXED>
 bool iterate_fits(const IterArgs &a)
 {
     constexpr int MOST = 180 * 1024;  // beside the static 16 KB
+    const int smem = iterate_smem<T>(a);
+    if (smem <= SMEM_UNASKED) return true;
     // asked for each time: the attribute belongs to the current context
     const bool ready = cudaFuncSetAttribute(k_iterate<T, MIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, MOST) ==
                        cudaSuccess;
     cudaGetLastError();
-    return ready && iterate_smem<T>(a) <= MOST;
+    return ready && smem <= MOST;
 }
 
 template <typename T, bool MIXED>
